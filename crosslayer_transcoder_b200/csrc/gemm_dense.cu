@@ -34,7 +34,7 @@ tc::TcOperand tc_operand(const Operand& o) {
 }
 
 SimtOperands simt_operands(const Operand& a, const Operand& b) {
-  SimtOperands s;
+  SimtOperands s{};
   s.A = (const float*)a.ptr;
   s.B = (const float*)b.ptr;
   s.sAz = a.mn * a.k;
@@ -53,7 +53,7 @@ int run_gemm(const GemmGeom& g, const Operand& a, const Operand& b, const typena
     CLT_CHECK_ARG(status != nullptr, "the tensor-core path needs a device status word");
     return tc::launch_gemm_tc<EpiBf16>(g, tc_operand(a), tc_operand(b), p16, status, device_sm_count(), stream);
   }
-  return launch_gemm_simt<EpiF32>(g, simt_operands(a, b), p32, stream);
+  return launch_gemm_simt<EpiF32>(g, simt_operands(a, b), p32, device_sm_count(), stream);
 }
 
 bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F > 0; }
