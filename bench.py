@@ -217,7 +217,7 @@ def algorithmic_work(spec, world: int, Fl: int, n_params: int, batch_bytes_per_e
         "clt_encoder_fwd_store[dead]": ("tensor", 2.0 * B * L * D * nd_pad),
         "clt_gather_enc_cols": ("hbm", float(L) * D * Fl * e + float(L) * D * nd_pad * e),
         "clt_encoder_dense_bwd_dw": ("tensor", 2.0 * B * L * D * Fd if spec.kind == "topk" else enc),
-        "clt_decoder_dense_fwd": ("tensor", dec), "clt_decoder_dense_fwd_push": ("tensor", dec),
+        "clt_decoder_dense_fwd_ws": ("tensor", dec), "clt_decoder_dense_fwd_push": ("tensor", dec),
         "clt_decoder_dense_bwd_dfeat": ("tensor", dec), "clt_decoder_dense_bwd_dw": ("tensor", dec),
         "clt_decoder_dense_bwd_dfeat_raw": ("tensor", dec),
         "clt_act_fwd": ("hbm", float(B) * L * Fl * e * 2), "clt_act_bwd": ("hbm", float(B) * L * Fl * e * 3),

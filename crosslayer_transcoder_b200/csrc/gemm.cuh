@@ -30,6 +30,7 @@ struct GemmGeom {
   int M, N, Kseg;  // slab shape and the length of one K-segment
   int L;           // number of layers (crosslayer modes)
   int nz;          // number of output slabs
+  int kb_per_part = 0;  // > 0: split-K, see below
 };
 
 __host__ __device__ inline int pair_index(int t, int s) { return t * (t + 1) / 2 + s; }
@@ -73,6 +74,48 @@ __host__ __device__ inline void seg_index(const GemmGeom& g, int z, int j, int& 
       za = z;
       zb = z;
   }
+}
+
+// Split-K.  The contraction of slab z, counted in the kernel's k-blocks (kb_per_seg to a segment), is cut into
+// parts of kb_per_part blocks, numbered slab by slab; part i writes its partial sums to output slab i.
+__host__ __device__ inline int part_count(const GemmGeom& g, int z, int kb_per_seg) {
+  return (seg_count(g, z) * kb_per_seg + g.kb_per_part - 1) / g.kb_per_part;
+}
+
+// What the work item of rank `rank` (0 .. nz-1) computes: operand slab z, its k-blocks [lo, hi), output slab zo.
+__host__ __device__ inline void work_item(const GemmGeom& g, int rank, int kb_per_seg, int& z, int& lo, int& hi,
+                                          int& zo) {
+  if (g.kb_per_part <= 0) {
+    z = zo = slab_of_rank(g, rank);
+    lo = 0;
+    hi = seg_count(g, z) * kb_per_seg;
+    return;
+  }
+  zo = rank;
+  z = 0;
+  int n;
+  while (rank >= (n = part_count(g, z, kb_per_seg))) rank -= n, ++z;
+  lo = rank * g.kb_per_part;
+  hi = seg_count(g, z) * kb_per_seg;
+  if (hi > lo + g.kb_per_part) hi = lo + g.kb_per_part;
+}
+
+// Blocks per part for a launch whose longest chain of k-blocks would outlast its fair share of the chip, 0 to
+// leave it whole.  `tiles` output tiles per slab run `slots` at a time, so a fair share is total * tiles / slots
+// blocks.  A chain may be 3/2 of that: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) the whole chains
+// took 170 us and parts 200 us; at 1.9 (fp32, 24 tiles, 1 to 12 segments of 64 blocks) 1784 and 1460 us; 9 tiles with
+// chains of 157 to 1884 blocks (12 calls) 4604 and 568 us.  Parts of half a share keep the last wave short; below
+// 8 blocks a part's output costs more than its products.
+inline int split_blocks(const GemmGeom& g, long long tiles, int kb_per_seg, int slots) {
+  long long total = 0, longest = 0;
+  for (int z = 0; z < g.nz; ++z) {
+    const long long n = (long long)seg_count(g, z) * kb_per_seg;
+    total += n;
+    longest = n > longest ? n : longest;
+  }
+  if (longest < 32 || longest * slots * 2 <= total * tiles * 3) return 0;
+  const long long part = (total * tiles + 2 * slots - 1) / (2 * slots);
+  return (int)(part < 8 ? 8 : part);
 }
 
 }  // namespace clt

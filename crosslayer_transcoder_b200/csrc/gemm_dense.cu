@@ -58,6 +58,39 @@ int run_gemm(const GemmGeom& g, const Operand& a, const Operand& b, const typena
 
 bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F > 0; }
 
+// recon[b, t, d] = b_dec[t, d] + the partial sums of target t's parts, in their order.  V consecutive d per thread.
+template <int V>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ ws, const float* __restrict__ b_dec,
+                                                        float* __restrict__ recon, GemmGeom g, int kb_per_seg) {
+  const int t = blockIdx.y;
+  const long long i = (blockIdx.x * 256ll + threadIdx.x) * V;
+  const long long slab = (long long)g.M * g.N;
+  if (i >= slab) return;
+  int first = 0;
+  for (int u = 0; u < t; ++u) first += part_count(g, u, kb_per_seg);
+  const int n = part_count(g, t, kb_per_seg);
+  const long long b = i / g.N;
+  const int d = (int)(i - b * g.N);
+  const float* p = ws + first * slab + i;
+  float acc[V];
+#pragma unroll
+  for (int q = 0; q < V; ++q) acc[q] = b_dec != nullptr ? __ldg(b_dec + (size_t)t * g.N + d + q) : 0.f;
+#pragma unroll 8
+  for (int j = 0; j < n; ++j) {
+    if (V == 4) {
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(p + j * slab));
+      acc[0] += v.x, acc[1 % V] += v.y, acc[2 % V] += v.z, acc[3 % V] += v.w;
+    } else {
+      acc[0] += __ldcs(p + j * slab);
+    }
+  }
+  float* o = recon + ((size_t)b * gridDim.y + t) * g.N + d;
+  if (V == 4)
+    *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1 % V], acc[2 % V], acc[3 % V]);
+  else
+    *o = acc[0];
+}
+
 }  // namespace
 
 extern "C" {
@@ -91,12 +124,46 @@ int clt_encoder_fwd_store(const void* xn, const void* W_enc, void* z_out, int B,
 
 int clt_decoder_dense_fwd(const void* feat, const void* W_dec, const float* b_dec, float* recon, int B, int L, int D,
                           int F, int crosslayer, int bf16, int* status, clt_stream_t stream) {
+  return clt_decoder_dense_fwd_ws(feat, W_dec, b_dec, recon, nullptr, 0, B, L, D, F, crosslayer, bf16, status, stream);
+}
+
+int clt_decoder_dense_fwd_ws(const void* feat, const void* W_dec, const float* b_dec, float* recon, float* ws,
+                             int64_t ws_floats, int B, int L, int D, int F, int crosslayer, int bf16, int* status,
+                             clt_stream_t stream) {
   CLT_CHECK_ARG(dims_ok(B, L, D, F), "decoder_dense_fwd: bad dims B=%d L=%d D=%d F=%d", B, L, D, F);
   CLT_CHECK_ARG(feat && W_dec && recon, "decoder_dense_fwd: null pointer");
   const int P = crosslayer ? L * (L + 1) / 2 : L;
   GemmGeom g{crosslayer ? kDecFwd : kBatched, B, D, F, L, L};
   Operand a{feat, 1, B, F, L}, b{W_dec, 0, D, F, P};
   epi::DecOut::Params p{recon, b_dec, (long long)L * D, (long long)D};
+  if (ws != nullptr) {
+    CLT_CHECK_ARG((uintptr_t)ws % 16 == 0, "decoder_dense_fwd: the workspace must be 16-byte aligned");
+    const int kb = bf16 ? tc::kBK : kSimtBK, kb_per_seg = (F + kb - 1) / kb;
+    // output tiles of a slab, and how many of them the chip works on at once (the fp32 kernel runs two to an SM)
+    const int bn = bf16 ? tc::kBN : 128;
+    const long long tiles = (long long)((B + 127) / 128) * ((D + bn - 1) / bn);
+    g.kb_per_part = split_blocks(g, tiles, kb_per_seg, device_sm_count() * (bf16 ? 1 : 2));
+    if (g.kb_per_part > 0) {
+      long long parts = 0;
+      for (int t = 0; t < L; ++t) parts += part_count(g, t, kb_per_seg);
+      if (parts * B * D <= ws_floats && parts <= 65535) {
+        g.nz = (int)parts;
+        epi::DecOut::Params pp{ws, nullptr, (long long)D, (long long)B * D};
+        if (int rc = run_gemm<epi::DecOut, epi::DecOut>(g, a, b, pp, pp, bf16, status, (cudaStream_t)stream)) return rc;
+        const long long slab = (long long)B * D;
+        if (D % 4 == 0 && ((uintptr_t)recon | (uintptr_t)b_dec) % 16 == 0) {
+          sum_parts_kernel<4><<<dim3((unsigned)((slab / 4 + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
+              ws, b_dec, recon, g, kb_per_seg);
+        } else {
+          sum_parts_kernel<1><<<dim3((unsigned)((slab + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
+              ws, b_dec, recon, g, kb_per_seg);
+        }
+        CLT_CHECK_CUDA(cudaGetLastError());
+        return 0;
+      }
+      g.kb_per_part = 0;  // the workspace is too small: whole chains
+    }
+  }
   return run_gemm<epi::DecOut, epi::DecOut>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
 }
 

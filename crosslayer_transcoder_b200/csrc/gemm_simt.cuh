@@ -131,7 +131,9 @@ __global__ void __launch_bounds__(kSimtThreads, 2) gemm_simt_kernel(GemmGeom g, 
   auto Bs = [&](int buf) { return smem + 2 * kSimtBK * TileA::kLd + buf * kSimtBK * TileB::kLd; };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int z = slab_of_rank(g, blockIdx.z);
+  const int kt_per_seg = (g.Kseg + kSimtBK - 1) / kSimtBK;
+  int zi, kt_lo, kt_hi, z;  // operand slab, its k-tiles, output slab
+  work_item(g, blockIdx.z, kt_per_seg, zi, kt_lo, kt_hi, z);
   const int m0 = blockIdx.y * BM;
   const int n0 = blockIdx.x * BN;
   // a warp covers 4 x 8 threads: its fragments are 64 and 128 contiguous bytes of a k-row
@@ -144,16 +146,15 @@ __global__ void __launch_bounds__(kSimtThreads, 2) gemm_simt_kernel(GemmGeom g, 
     for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
 
   const bool kcA = op.sAk == 1, kcB = op.sBk == 1;
-  const int kt_per_seg = (g.Kseg + kSimtBK - 1) / kSimtBK;
-  const int n_kt = seg_count(g, z) * kt_per_seg;
+  const int n_kt = kt_hi - kt_lo;
   TileA ta;
   TileB tb;
-  int seg = 0, kt = 0;  // the k-tile to be loaded next
+  int seg = kt_lo / kt_per_seg, kt = kt_lo % kt_per_seg;  // the k-tile to be loaded next
   const float *Ap = nullptr, *Bp = nullptr;
   auto load_next = [&]() {
-    if (kt == 0) {
+    if (kt == 0 || Ap == nullptr) {
       int za, zb;
-      seg_index(g, z, seg, za, zb);
+      seg_index(g, zi, seg, za, zb);
       Ap = op.A + (long long)za * op.sAz;
       Bp = op.B + (long long)zb * op.sBz;
     }

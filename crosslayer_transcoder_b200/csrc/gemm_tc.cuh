@@ -247,15 +247,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         uint32_t phase = 0;
         bool alive = true;
         for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x) {
-          const int z = slab_of_rank(g, tile / tiles_per_slab);
+          int z, kb_lo, kb_hi, zo;
+          work_item(g, tile / tiles_per_slab, kb_per_seg, z, kb_lo, kb_hi, zo);
           const int r = tile % tiles_per_slab;
           int m0, n0;
           tile_origin(r, m_tiles, n_tiles, m0, n0);
-          const int nseg = seg_count(g, z);
-          for (int j = 0; j < nseg && alive; ++j) {
+          int left = kb_hi - kb_lo, kb0 = kb_lo % kb_per_seg;
+          for (int j = kb_lo / kb_per_seg; left > 0 && alive; ++j) {
             int za, zb;
             seg_index(g, z, j, za, zb);
-            for (int kb = 0; kb < kb_per_seg; ++kb) {
+            const int kb1 = min(kb_per_seg, kb0 + left);
+            left -= kb1 - kb0;
+            for (int kb = kb0; kb < kb1; ++kb) {
               if (!mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1, abort_flag, status, kTimeoutEmpty)) {
                 alive = false;
                 break;
@@ -279,6 +282,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
               }
               if (++stage == kStages) stage = 0, phase ^= 1;
             }
+            kb0 = 0;
           }
         }
         if (!alive) {
@@ -300,8 +304,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         bool alive = true;
         for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x, ++it) {
           const int buf = it & 1;
-          const int z = slab_of_rank(g, tile / tiles_per_slab);
-          const int nkb = seg_count(g, z) * kb_per_seg;
+          int z, kb_lo, kb_hi, zo;
+          work_item(g, tile / tiles_per_slab, kb_per_seg, z, kb_lo, kb_hi, zo);
+          const int nkb = kb_hi - kb_lo;
           if (!mbar_wait(smem_u32(&bars->tmem_empty[buf]), acc_phase[buf] ^ 1, abort_flag, status, kTimeoutTmemEmpty))
             break;
           acc_phase[buf] ^= 1;
@@ -344,7 +349,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     int it = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
       const int buf = it & 1;
-      const int z = slab_of_rank(g, tile / tiles_per_slab);
+      int zi, kb_lo, kb_hi, z;  // z: the output slab
+      work_item(g, tile / tiles_per_slab, kb_per_seg, zi, kb_lo, kb_hi, z);
       const int r = tile % tiles_per_slab;
       int m0, n0;
       tile_origin(r, m_tiles, n_tiles, m0, n0);

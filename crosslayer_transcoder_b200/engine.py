@@ -396,6 +396,19 @@ class StepEngine:
         lists and for rows too wide for one warp's registers."""
         return int(k <= 8 * world or (k <= 64 and D <= 1024))
 
+    def _decoder_dense_fwd(self, feat, W, bias, recon, B, L, D, F, crosslayer, bf16):
+        """The dense decoder contraction, with scratch for partial sums where the library may want to split the
+        contraction axis (csrc/gemm.cuh, ``split_blocks``: at most two parts per running tile, and one rounded
+        up per target).  The scratch is this call's own: forwards may run on several streams."""
+        tiles = -(-B // 128) * -(-D // (256 if bf16 else 128))
+        slots = 148 if bf16 else 296
+        ws, n = None, 0
+        if 4 * slots > 3 * (L + 1) * tiles:
+            n = (2 * slots // tiles + L + 1) * B * D
+            ws = torch.empty(n, dtype=torch.float32, device=recon.device)
+        self._call("clt_decoder_dense_fwd_ws", feat, W, bias, recon, ws, n, B, L, D, F, crosslayer, int(bf16),
+                   self.status, stream_ptr())
+
     def _rank_barrier(self, px):
         """Order the ranks on the compute stream: a one-element all-reduce.  After it, every kernel that
         any rank enqueued before its own call has finished, so rows pushed into this rank's buffers
@@ -489,8 +502,7 @@ class StepEngine:
                            acc[2:4], b_cnt, L, D, s)
             all_reduce_sum(acc[0:4], group)             # encoder-side sums of all shards, loss sums of all owners
         else:
-            self._call("clt_decoder_dense_fwd", feat, W_op, dec.b.data if first_rank else None, recon, B, L, D, F,
-                       crosslayer, int(bf16), self.status, s)
+            self._decoder_dense_fwd(feat, W_op, dec.b.data if first_rank else None, recon, B, L, D, F, crosslayer, bf16)
             if world > 1:
                 from .parallel import all_reduce_sum
 
@@ -565,8 +577,7 @@ class StepEngine:
             theta = nl.theta.data if kind == "jumprelu" else None
             self._call("clt_act_fwd", z, enc.b.data, theta, None, feat, None, scratch, 1.0, 0, 0, B, L, F, int(bf16), s)
             self._call("clt_export_blf", feat, None, features, B, L, F, int(bf16), s)
-            self._call("clt_decoder_dense_fwd", feat, W_op, bias, recon, B, L, D, F, crosslayer, int(bf16),
-                       self.status, s)
+            self._decoder_dense_fwd(feat, W_op, bias, recon, B, L, D, F, crosslayer, bf16)
             if world > 1:
                 from .parallel import all_reduce_sum
 
@@ -658,8 +669,7 @@ class StepEngine:
         w_op = self._operand(w, bf16)
         w_op = w_op.reshape(1, K, D) if dec.crosslayer else w_op[layer:layer + 1]
         recon = torch.empty(B, 1, D, dtype=torch.float32, device=dev)
-        self._call("clt_decoder_dense_fwd", feat, w_op, dec.b.data[layer:layer + 1], recon, B, 1, D, K, 0, int(bf16),
-                   self.status, s)
+        self._decoder_dense_fwd(feat, w_op, dec.b.data[layer:layer + 1], recon, B, 1, D, K, 0, bf16)
         return recon.reshape(*lead, D)
 
     # ------------------------------------------------------------------ backward
@@ -894,8 +904,7 @@ class StepEngine:
                 self._call("clt_decoder_dense_fwd_push", a_aux, w_c, bias, px["aux_bases"], px["rpr"], world,
                            mod.tp_rank, px["slot_bf16"], B, L, D, nd_pad, crosslayer, int(bf16), self.status, s)
             else:
-                self._call("clt_decoder_dense_fwd", a_aux, w_c, bias, aux_recon, B, L, D, nd_pad, crosslayer,
-                           int(bf16), self.status, s)
+                self._decoder_dense_fwd(a_aux, w_c, bias, aux_recon, B, L, D, nd_pad, crosslayer, bf16)
             aux = dict(dead_list=dead_list, n_dead=n_dead, nd_pad=nd_pad, a_aux=a_aux, w_c=w_c)
             if world > 1 and px is None:
                 pending.append(all_reduce_sum(rbuf[n_rec:2 * n_rec], group, async_op=True))
