@@ -9,48 +9,159 @@
 namespace clt {
 namespace {
 
+// Rows of V consecutive elements in registers; V = 8 needs rows that start on 16-byte boundaries.
+template <class T, int V>
+__device__ __forceinline__ void load_row(const T* p, float (&o)[V]) {
+  if constexpr (V == 1) {
+    if constexpr (sizeof(T) == 2)
+      o[0] = __bfloat162float(*p);
+    else
+      o[0] = *p;
+  } else if constexpr (sizeof(T) == 2) {
+    const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p));
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      o[2 * j] = __uint_as_float(w[j] << 16);
+      o[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float4 t = __ldcs(reinterpret_cast<const float4*>(p) + j);
+      o[4 * j] = t.x, o[4 * j + 1] = t.y, o[4 * j + 2] = t.z, o[4 * j + 3] = t.w;
+    }
+  }
+}
+template <class T, int V>
+__device__ __forceinline__ void store_row(T* p, const float (&v)[V]) {
+  if constexpr (V == 1) {
+    if constexpr (sizeof(T) == 2)
+      *p = __float2bfloat16_rn(v[0]);
+    else
+      *p = v[0];
+  } else if constexpr (sizeof(T) == 2) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                              pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      reinterpret_cast<float4*>(p)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
+}
 template <class T>
-__device__ __forceinline__ float cvt_in(T v);
-template <>
-__device__ __forceinline__ float cvt_in<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float cvt_in<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float rounded(float x) {
+  return sizeof(T) == 2 ? bf16_round(x) : x;
+}
+
+// The three layout kernels below are bound by HBM.  A CTA covers 256 V columns of one layer (blockIdx.x, blockIdx.z) and
+// walks batch rows (blockIdx.y strided), so an element costs no division and the per-column parameters stay in
+// registers; V = 8 makes every access 16 bytes wide.  export at [12, 1000, 10000] bf16: 472 -> 162 us (4.4 TB/s), one
+// element per thread and step with two 64-bit divisions before; act_export at [12, 333, 24576] 228 us (5.2 TB/s) for what
+// an activation sweep and two exports took 900 us.
 
 // out[b, l, f] = src[l, b, f] (+ bias[l, f])     layer-major T -> token-major fp32
-template <class T>
-__global__ void export_blf_kernel(const T* __restrict__ src, const float* __restrict__ bias, float* __restrict__ out,
-                                  int B, int L, long long F) {
-  const long long total = (long long)B * L * F;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long f = i % F;
-    const long long r = i / F;
-    const int l = (int)(r % L);
-    const long long b = r / L;
-    float v = cvt_in<T>(src[((long long)l * B + b) * F + f]);
-    if (bias != nullptr) v += __ldg(bias + (long long)l * F + f);
-    out[i] = v;
+template <class T, int V>
+__global__ void __launch_bounds__(256)
+export_blf_kernel(const T* __restrict__ src, const float* __restrict__ bias, float* __restrict__ out, int B, int L,
+                  long long F) {
+  const long long f = (blockIdx.x * 256ll + threadIdx.x) * V;
+  const int l = blockIdx.z;
+  if (f >= F) return;
+  float bb[V];
+#pragma unroll
+  for (int q = 0; q < V; ++q) bb[q] = 0.f;
+  if (bias != nullptr) {
+#pragma unroll
+    for (int q = 0; q < V; ++q) bb[q] = __ldg(bias + l * F + f + q);
+  }
+#pragma unroll 2
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    float v[V];
+    load_row<T, V>(src + ((long long)l * B + b) * F + f, v);
+    if (bias != nullptr) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) v[q] += bb[q];
+    }
+    store_row<float, V>(out + ((long long)b * L + l) * F + f, v);
   }
 }
 
-// dst[l, b, f] = T(src[b, l, f])                  token-major fp32 -> layer-major T
-template <class T>
-__global__ void import_blf_kernel(const float* __restrict__ src, T* __restrict__ dst, int B, int L, long long F) {
-  const long long total = (long long)B * L * F;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long f = i % F;
-    const long long r = i / F;
-    const int l = (int)(r % L);
-    const long long b = r / L;
-    const float v = src[i];
-    if constexpr (sizeof(T) == 2)
-      dst[((long long)l * B + b) * F + f] = __float2bfloat16_rn(v);
-    else
-      dst[((long long)l * B + b) * F + f] = v;
+// pre[b, l, f] = z[l, b, f] + bias[l, f];  feat[l, b, f] = T(pre [pre > theta, pre > 0]);  features[b, l, f] = feat:
+// the validation forward's (Jump)ReLU and both of its token-major outputs from one sweep of z
+template <class T, int V>
+__global__ void __launch_bounds__(256)
+act_export_kernel(const T* __restrict__ z, const float* __restrict__ bias, const float* __restrict__ theta,
+                  float* __restrict__ pre, T* __restrict__ feat, float* __restrict__ features, int B, int L,
+                  long long F) {
+  const long long f = (blockIdx.x * 256ll + threadIdx.x) * V;
+  const int l = blockIdx.z;
+  if (f >= F) return;
+  float bb[V], tt[V];
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    bb[q] = __ldg(bias + l * F + f + q);
+    tt[q] = theta != nullptr ? __ldg(theta + l * F + f + q) : 0.f;
+  }
+#pragma unroll 2
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    const long long lm = ((long long)l * B + b) * F + f, tm = ((long long)b * L + l) * F + f;
+    float v[V], a[V];
+    load_row<T, V>(z + lm, v);
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      v[q] += bb[q];
+      a[q] = rounded<T>(v[q] > tt[q] && v[q] > 0.f ? v[q] : 0.f);
+    }
+    store_row<float, V>(pre + tm, v);
+    store_row<T, V>(feat + lm, a);
+    store_row<float, V>(features + tm, a);
   }
 }
 
+// dst[l, b, f] = T(src[b * ld + l * F + f])       fp32 rows of any distance -> layer-major T
+template <class T, int V>
+__global__ void __launch_bounds__(256)
+import_rows_kernel(const float* __restrict__ src, long long ld, T* __restrict__ dst, int B, long long F) {
+  const long long f = (blockIdx.x * 256ll + threadIdx.x) * V;
+  const int l = blockIdx.z;
+  if (f >= F) return;
+#pragma unroll 2
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    float v[V];
+    load_row<float, V>(src + (long long)b * ld + l * F + f, v);
+    store_row<T, V>(dst + ((long long)l * B + b) * F + f, v);
+  }
+}
+
+// grid of the kernels above: about 16 CTAs per SM, fewer rows per CTA rather than fewer CTAs
+inline dim3 row_grid(int B, int L, long long F, int V) {
+  const long long gx = (F + 256ll * V - 1) / (256ll * V);
+  long long gy = (148ll * 16 + gx * L - 1) / (gx * L);
+  if (gy > B) gy = B;
+  return dim3((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535), (unsigned)L);
+}
+inline bool aligned16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
+  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d) & 15) == 0;
+}
+template <class T>
+int launch_import(const float* src, long long ld, void* dst, int B, int L, long long F, cudaStream_t s) {
+  if (F % 8 == 0 && ld % 4 == 0 && aligned16(src, dst))
+    import_rows_kernel<T, 8><<<row_grid(B, L, F, 8), 256, 0, s>>>(src, ld, (T*)dst, B, F);
+  else
+    import_rows_kernel<T, 1><<<row_grid(B, L, F, 1), 256, 0, s>>>(src, ld, (T*)dst, B, F);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+template <class T>
+int launch_export(const void* src, const float* bias, float* out, int B, int L, long long F, cudaStream_t s) {
+  if (F % 8 == 0 && aligned16(src, out))
+    export_blf_kernel<T, 8><<<row_grid(B, L, F, 8), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
+  else
+    export_blf_kernel<T, 1><<<row_grid(B, L, F, 1), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
 // out[b, l, d] = recon[b, l, d] * sd[l, d] + mu[l, d]
 __global__ void destandardize_kernel(const float* __restrict__ recon, const float* __restrict__ mu,
                                      const float* __restrict__ sd, float* __restrict__ out, long long total, int LD) {
@@ -103,27 +214,39 @@ int clt_prep_acts(const void* acts, int in_dtype, const float* mu, const float* 
 
 int clt_export_blf(const void* src, const float* bias, float* out, int B, int L, int64_t F, int bf16,
                    clt_stream_t stream) {
-  CLT_CHECK_ARG(src && out && B > 0 && L > 0 && F > 0, "export_blf: bad arguments");
-  const long long total = (long long)B * L * F;
+  CLT_CHECK_ARG(src && out && B > 0 && L > 0 && L <= 65535 && F > 0, "export_blf: bad arguments");
+  return bf16 ? launch_export<__nv_bfloat16>(src, bias, out, B, L, F, (cudaStream_t)stream)
+              : launch_export<float>(src, bias, out, B, L, F, (cudaStream_t)stream);
+}
+
+int clt_act_export(const void* z, const float* bias, const float* theta, float* pre, void* feat, float* features, int B,
+                   int L, int64_t F, int bf16, clt_stream_t stream) {
+  CLT_CHECK_ARG(z && bias && pre && feat && features && B > 0 && L > 0 && L <= 65535 && F > 0,
+                "act_export: bad arguments");
+  CLT_CHECK_ARG(F % 8 == 0, "act_export: d_features=%lld must be a multiple of 8", (long long)F);
+  CLT_CHECK_ARG(aligned16(z, pre, feat, features), "act_export: buffers must be 16-byte aligned");
+  const dim3 grid = row_grid(B, L, F, 8);
   cudaStream_t s = (cudaStream_t)stream;
   if (bf16)
-    export_blf_kernel<__nv_bfloat16><<<grid_for(total), 256, 0, s>>>((const __nv_bfloat16*)src, bias, out, B, L, F);
+    act_export_kernel<__nv_bfloat16, 8><<<grid, 256, 0, s>>>((const __nv_bfloat16*)z, bias, theta, pre,
+                                                             (__nv_bfloat16*)feat, features, B, L, F);
   else
-    export_blf_kernel<float><<<grid_for(total), 256, 0, s>>>((const float*)src, bias, out, B, L, F);
+    act_export_kernel<float, 8><<<grid, 256, 0, s>>>((const float*)z, bias, theta, pre, (float*)feat, features, B, L, F);
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
 int clt_import_blf(const float* src, void* dst, int B, int L, int64_t F, int bf16, clt_stream_t stream) {
-  CLT_CHECK_ARG(src && dst && B > 0 && L > 0 && F > 0, "import_blf: bad arguments");
-  const long long total = (long long)B * L * F;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (bf16)
-    import_blf_kernel<__nv_bfloat16><<<grid_for(total), 256, 0, s>>>(src, (__nv_bfloat16*)dst, B, L, F);
-  else
-    import_blf_kernel<float><<<grid_for(total), 256, 0, s>>>(src, (float*)dst, B, L, F);
-  CLT_CHECK_CUDA(cudaGetLastError());
-  return 0;
+  CLT_CHECK_ARG(src && dst && B > 0 && L > 0 && L <= 65535 && F > 0, "import_blf: bad arguments");
+  const long long ld = (long long)L * F;
+  return bf16 ? launch_import<__nv_bfloat16>(src, ld, dst, B, L, F, (cudaStream_t)stream)
+              : launch_import<float>(src, ld, dst, B, L, F, (cudaStream_t)stream);
+}
+
+int clt_import_rows(const float* src, int64_t ld, void* dst, int rows, int64_t K, int bf16, clt_stream_t stream) {
+  CLT_CHECK_ARG(src && dst && rows > 0 && K > 0 && ld >= 0, "import_rows: bad arguments");
+  return bf16 ? launch_import<__nv_bfloat16>(src, ld, dst, rows, 1, K, (cudaStream_t)stream)
+              : launch_import<float>(src, ld, dst, rows, 1, K, (cudaStream_t)stream);
 }
 
 int clt_destandardize(const float* recon, const float* mu, const float* sd, float* out, int B, int L, int D,

@@ -565,7 +565,8 @@ class StepEngine:
         z = torch.empty(L, B, F, dtype=T, device=dev)
         self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16), z, B, L, D, F, int(bf16), self.status, s)
         pre_actvs = torch.empty(B, L, F, dtype=torch.float32, device=dev)
-        self._call("clt_export_blf", z, enc.b.data, pre_actvs, B, L, F, int(bf16), s)
+        if kind not in ("jumprelu", "relu"):
+            self._call("clt_export_blf", z, enc.b.data, pre_actvs, B, L, F, int(bf16), s)
         features = torch.empty(B, L, F, dtype=torch.float32, device=dev)
         recon = torch.empty(B, L, D, dtype=torch.float32, device=dev)
         W_op, _, _ = self._dec_flat(bf16)
@@ -573,10 +574,8 @@ class StepEngine:
         bias = dec.b.data if getattr(mod, "tp_rank", 0) == 0 else None
         if kind in ("jumprelu", "relu"):
             feat = torch.empty(L, B, F, dtype=T, device=dev)
-            scratch = torch.zeros(2, dtype=torch.float32, device=dev)
             theta = nl.theta.data if kind == "jumprelu" else None
-            self._call("clt_act_fwd", z, enc.b.data, theta, None, feat, None, scratch, 1.0, 0, 0, B, L, F, int(bf16), s)
-            self._call("clt_export_blf", feat, None, features, B, L, F, int(bf16), s)
+            self._call("clt_act_export", z, enc.b.data, theta, pre_actvs, feat, features, B, L, F, int(bf16), s)
             self._decoder_dense_fwd(feat, W_op, bias, recon, B, L, D, F, crosslayer, bf16)
             if world > 1:
                 from .parallel import all_reduce_sum
@@ -657,7 +656,9 @@ class StepEngine:
             n_src, lead = 1, features.shape[:-1]
             w = dec.W
         K = n_src * F
-        x = features.reshape(-1, K).float().contiguous()
+        x = features.reshape(-1, K).float()          # a view of the sources 0..layer keeps the distance of its rows
+        if x.stride(1) != 1:
+            x = x.contiguous()
         B = x.shape[0]
         bf16 = self._precision(x)
         dev = x.device
@@ -665,7 +666,7 @@ class StepEngine:
         T = torch.bfloat16 if bf16 else torch.float32
         s = stream_ptr()
         feat = torch.empty(1, B, K, dtype=T, device=dev)
-        self._call("clt_import_blf", x, feat, B, 1, K, int(bf16), s)
+        self._call("clt_import_rows", x, x.stride(0), feat, B, K, int(bf16), s)
         w_op = self._operand(w, bf16)
         w_op = w_op.reshape(1, K, D) if dec.crosslayer else w_op[layer:layer + 1]
         recon = torch.empty(B, 1, D, dtype=torch.float32, device=dev)

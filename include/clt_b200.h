@@ -386,7 +386,11 @@ int clt_batchtopk_threshold_update(uint64_t* state, float* threshold, float e, i
  * layer-major operands.
  * clt_prep_acts: xn[l,b,:] = T((acts[b,l,:] - mu[l]) / sd[l]) for acts [B, L, D] (mu = sd = NULL: cast only).
  * clt_export_blf: out[b,l,:] = src[l,b,:] (+ bias[l,:]), src [L, B, F] in T, out [B, L, F] fp32.
+ * clt_act_export: the (Jump)ReLU of the stored contraction output z [L, B, F] with both token-major fp32 results:
+ *   pre[b,l,:] = z[l,b,:] + bias[l,:];  feat[l,b,:] = T(pre where pre > theta[l,:] and pre > 0, else 0);
+ *   features[b,l,:] = feat[l,b,:].  theta may be NULL (ReLU).
  * clt_import_blf: dst[l,b,:] = T(src[b,l,:]).
+ * clt_import_rows: dst[r,:] = T(src[r * ld + ...]), rows of K elements at any distance ld.
  * clt_destandardize: out = recon * sd + mu (DimensionwiseOutputStandardizer.forward, standardize.py:88-98).
  * clt_scatter_features: dense [B, L, F] fp32 zeroed, then dense[token(e), l, idx[e]] = val[e] for the valid
  * entries of the lists idx / val [L, npl] (etok NULL: token = slot / k, npl = B k). */
@@ -394,6 +398,9 @@ int clt_prep_acts(const void* acts, int in_dtype, const float* mu, const float* 
                   int L, int D, clt_stream_t stream);
 int clt_export_blf(const void* src, const float* bias, float* out, int B, int L, int64_t F, int bf16,
                    clt_stream_t stream);
+int clt_act_export(const void* z, const float* bias, const float* theta, float* pre, void* feat, float* features, int B,
+                   int L, int64_t F, int bf16, clt_stream_t stream);
+int clt_import_rows(const float* src, int64_t ld, void* dst, int rows, int64_t K, int bf16, clt_stream_t stream);
 int clt_import_blf(const float* src, void* dst, int B, int L, int64_t F, int bf16, clt_stream_t stream);
 int clt_destandardize(const float* recon, const float* mu, const float* sd, float* out, int B, int L, int D,
                       clt_stream_t stream);

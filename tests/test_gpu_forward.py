@@ -96,3 +96,33 @@ def test_forward_layer_runs_on_the_kernels(cross, prec):
     assert mod._engine.launches >= n0 + 10      # 2 layers x (3 encoder-side + 2 decoder-side) launches
     mod._engine.check_status("forward_layer")
     assert torch.equal(enc.cpu()(x.cpu(), layer=0), x.cpu() @ enc.W[0] + enc.b[0])      # CPU tensors: eager definition
+
+
+@pytest.mark.parametrize("bf16", [0, 1])
+@pytest.mark.parametrize("L,B,F", [(1, 1, 8), (3, 7, 2048), (2, 5, 2056), (3, 4, 77), (2, 3000, 24)])
+def test_layout_kernels(L, B, F, bf16):
+    """Token-major <-> layer-major copies at the ends of their column blocks, for rows that do and do not start on
+    16 bytes, from strided sources too: bit for bit."""
+    from crosslayer_transcoder_b200._lib import lib, stream_ptr
+
+    dev, T = "cuda:0", torch.bfloat16 if bf16 else torch.float32
+    g = torch.Generator(device=dev).manual_seed(B + F)
+    z = torch.randn(L, B, F, generator=g, device=dev).to(T)
+    bias, theta = torch.randn(L, F, generator=g, device=dev), torch.rand(L, F, generator=g, device=dev) * 0.5
+    pre = z.float().transpose(0, 1) + bias
+    out = torch.empty(B, L, F, device=dev)
+    lib().call("clt_export_blf", z, bias, out, B, L, F, bf16, stream_ptr())
+    assert torch.equal(out, pre)
+    back = torch.empty_like(z)
+    lib().call("clt_import_blf", out, back, B, L, F, bf16, stream_ptr())
+    assert torch.equal(back, pre.transpose(0, 1).to(T))
+    for n, wide in ((1, out), (L, torch.randn(B, L + 1, F, generator=g, device=dev))):      # sources 0..n-1 of wider rows
+        x = wide[:, :n].reshape(B, n * F)
+        rows = torch.empty(B, n * F, dtype=T, device=dev)
+        lib().call("clt_import_rows", x, x.stride(0), rows, B, n * F, bf16, stream_ptr())
+        assert torch.equal(rows, x.to(T))
+    if F % 8 == 0:
+        want = torch.where((pre > theta) & (pre > 0), pre, torch.zeros_like(pre)).to(T)
+        p2, f2, feat = torch.empty_like(out), torch.empty_like(out), torch.empty_like(z)
+        lib().call("clt_act_export", z, bias, theta, p2, feat, f2, B, L, F, bf16, stream_ptr())
+        assert torch.equal(p2, pre) and torch.equal(f2, want.float()) and torch.equal(feat, want.transpose(0, 1))
