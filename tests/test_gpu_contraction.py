@@ -83,3 +83,43 @@ def test_split_decoder(L, B, D, F, cross, bf16):
         want = torch.einsum("sbf,sfd->bd", fd, wd) + b[t].double()
         mag = torch.einsum("sbf,sfd->bd", fd.abs(), wd.abs()) + b[t].double().abs()
         _close(split[:, t], want, mag, fd.shape[0] * F)
+
+
+# 256-row tiles of CTA pairs (the batch large enough, rounding it up to 256 rows cheap) and 128-row tiles, with ragged
+# ends in every axis; a contraction of a few elements, one of one stage, one of more stages than the ring holds
+@pytest.mark.parametrize("L,B,D,F", [(2, 2049, 264, 2056), (1, 4000, 776, 3000), (3, 1281, 8, 4104), (3, 1100, 64, 2312),
+                                     (2, 300, 520, 1032), (12, 256, 256, 2048)])
+def test_bf16_products(L, B, D, F):
+    dev = "cuda:0"
+    g = torch.Generator(device=dev).manual_seed(B)
+    s, st = stream_ptr(), torch.zeros(1, dtype=torch.int32, device=dev)
+    bf = torch.bfloat16
+    P = L * (L + 1) // 2
+    x, W, feat, dr = (_rand(g, *n).to(bf) for n in ((L, B, D), (L, D, F), (L, B, F), (L, B, D)))
+    Wd, b = _rand(g, P, F, D).to(bf), _rand(g, L, D)
+
+    def rounded(got, want, mag, k):
+        """a bf16 result is its fp32 sum rounded once more"""
+        bound = 2.0 ** -24 * (4.0 + 2.0 * k ** 0.5) * mag + 2.0 ** -8 * want.abs() + 1e-30
+        assert bool(((got.double() - want).abs() <= bound).all()), float(((got.double() - want).abs() / bound).max())
+
+    z, df = torch.empty(L, B, F, device=dev, dtype=bf), torch.empty(L, B, F, device=dev, dtype=bf)
+    lib().call("clt_encoder_fwd_store", x, W, z, B, L, D, F, 1, st, s)
+    lib().call("clt_decoder_dense_bwd_dfeat_raw", dr, Wd, df, B, L, D, F, 1, 1, st, s)
+    recon = torch.empty(B, L, D, device=dev)
+    lib().call("clt_decoder_dense_fwd", feat, Wd, b, recon, B, L, D, F, 1, 1, st, s)
+    dW, dWe = torch.empty(P, F, D, device=dev), torch.empty(L, D, F, device=dev)
+    lib().call("clt_decoder_dense_bwd_dw", feat, dr, dW, None, None, B, L, D, F, 1, 1, st, s)
+    lib().call("clt_encoder_dense_bwd_dw", x, feat, dWe, B, L, D, F, 1, st, s)
+    assert int(st) == 0
+    mm = lambda a, w: (a.double() @ w.double(), a.double().abs() @ w.double().abs())
+    for l in range(L):
+        rounded(z[l], *mm(x[l], W[l]), D)
+        _close(dWe[l], *mm(x[l].t(), feat[l]), B)
+        blk = Wd[l * (l + 1) // 2:(l + 1) * (l + 2) // 2].reshape(-1, D)
+        want, mag = mm(feat[:l + 1].transpose(0, 1).reshape(B, -1), blk)
+        _close(recon[:, l], want + b[l].double(), mag + b[l].double().abs(), (l + 1) * F)
+        for q in range(l + 1):
+            _close(dW[l * (l + 1) // 2 + q], *mm(feat[q].t(), dr[l]), B)
+        blk = torch.cat([Wd[t * (t + 1) // 2 + l] for t in range(l, L)], dim=1)
+        rounded(df[l], *mm(dr[l:].transpose(0, 1).reshape(B, -1), blk.t()), (L - l) * D)
