@@ -55,9 +55,18 @@ class FlatParams:
                 view = self.view_of(p, self.flat)
                 view.copy_(p.data)
                 p.data = view
+        self._bytes = [4 * self.offsets[id(p)] for p in self.params]
         self._shadow_version = None
+        self._operands: Dict[int, torch.Tensor] = {}
         if want_bf16:
             self.ensure_shadow()
+
+    def operand(self, p: torch.nn.Parameter) -> torch.Tensor:
+        """``p``'s slice of the bf16 copy."""
+        v = self._operands.get(id(p))
+        if v is None:
+            v = self._operands[id(p)] = self.view_of(p, self.shadow)
+        return v
 
     def view_of(self, p: torch.nn.Parameter, buf: torch.Tensor) -> torch.Tensor:
         o = self.offsets[id(p)]
@@ -65,16 +74,20 @@ class FlatParams:
 
     def is_packed(self) -> bool:
         base = self.flat.data_ptr()
-        return all(p.data_ptr() == base + 4 * self.offsets[id(p)] for p in self.params)
+        for p, o in zip(self.params, self._bytes):
+            if p.data_ptr() != base + o:
+                return False
+        return True
 
     def _version(self):
-        return tuple(p._version for p in self.params)
+        return [p._version for p in self.params]
 
     def ensure_shadow(self):
         """(Re)build the bf16 copy when parameters were changed by anything but the fused Adam step."""
         v = self._version()
         if self.shadow is None:
             self.shadow = torch.empty(self.numel, dtype=torch.bfloat16, device=self.device)
+            self._operands.clear()
             self._shadow_version = None
         if self._shadow_version != v:
             lib().call("clt_cast_bf16", self.flat, self.shadow, self.numel, stream_ptr())
@@ -95,7 +108,7 @@ class _Workspace:
 
     def get(self, name, shape, dtype, device, zero=False):
         t = self.buf.get(name)
-        if t is None or t.shape != torch.Size(shape) or t.dtype != dtype or t.device != device:
+        if t is None or t.shape != shape or t.dtype != dtype or t.device != device:
             t = (torch.zeros if zero else torch.empty)(shape, dtype=dtype, device=device)
             self.buf[name] = t
         return t
@@ -222,7 +235,7 @@ class StepEngine:
     # ------------------------------------------------------------------ helpers
     def _operand(self, p: torch.nn.Parameter, bf16: bool) -> torch.Tensor:
         """The tensor a contraction reads for parameter ``p``: its bf16 copy or the fp32 master."""
-        return self.flat.view_of(p, self.flat.shadow) if bf16 else p.data
+        return self.flat.operand(p) if bf16 else p.data
 
     def _dec_flat(self, bf16: bool):
         """(operand buffer [P,F,D], fp32 master [P,F,D], gradient [P,F,D]) of the decoder blocks;
@@ -250,7 +263,7 @@ class StepEngine:
             raise CltError("the fused step needs both standardizers")
         if not (ins.is_initialized and outs.is_initialized):
             raise ValueError("Standardizer not initialized")
-        f = lambda t: t.detach().float().contiguous()
+        f = lambda t: t if t.dtype == torch.float32 and t.is_contiguous() else t.detach().float().contiguous()
         return f(ins.mean), f(ins.std), f(outs.mean), f(outs.std)
 
     def _fuse_activation(self, D: int, F: int, bf16: bool) -> bool:
@@ -275,9 +288,10 @@ class StepEngine:
         """``idxs_dead.float().mean()`` of the last step (reference clt_lightning.py:286-287) as a device
         scalar; on feature shards the mean over all shards."""
         enc = self.module.model.encoder
-        cnt = self._dead_cnt.to(torch.float32)
+        cnt = self._dead_cnt
         world = getattr(self.module, "tp_world", 1)
         if world > 1:
+            cnt = cnt.to(torch.float32)
             from .parallel import all_reduce_sum
 
             all_reduce_sum(cnt, self.module.tp_group)
@@ -396,14 +410,14 @@ class StepEngine:
         lists and for rows too wide for one warp's registers."""
         return int(k <= 8 * world or (k <= 64 and D <= 1024))
 
-    def _decoder_dense_fwd(self, feat, W, bias, recon, B, L, D, F, crosslayer, bf16):
+    def _decoder_dense_fwd(self, feat, W, bias, recon, B, L, D, F, crosslayer, bf16, split=True):
         """The dense decoder contraction, with scratch for partial sums where the library may want to split the
         contraction axis (csrc/gemm.cuh, ``split_blocks``: at most two parts per running tile, and one rounded
         up per target).  The scratch is this call's own: forwards may run on several streams."""
         tiles = -(-B // 128) * -(-D // (256 if bf16 else 128))
         slots = 148 if bf16 else 296
         ws, n = None, 0
-        if 4 * slots > 3 * (L + 1) * tiles:
+        if split and 4 * slots > 3 * (L + 1) * tiles:
             n = (2 * slots // tiles + L + 1) * B * D
             ws = torch.empty(n, dtype=torch.float32, device=recon.device)
         self._call("clt_decoder_dense_fwd_ws", feat, W, bias, recon, ws, n, B, L, D, F, crosslayer, int(bf16),
@@ -502,7 +516,10 @@ class StepEngine:
                            acc[2:4], b_cnt, L, D, s)
             all_reduce_sum(acc[0:4], group)             # encoder-side sums of all shards, loss sums of all owners
         else:
-            self._decoder_dense_fwd(feat, W_op, dec.b.data if first_rank else None, recon, B, L, D, F, crosslayer, bf16)
+            # bf16: whole chains whatever the batch.  Partial sums round differently, and in a small batch a
+            # (Jump)ReLU gradient can hang on one pre-activation that falls on the other side for it.
+            self._decoder_dense_fwd(feat, W_op, dec.b.data if first_rank else None, recon, B, L, D, F, crosslayer, bf16,
+                                    split=not bf16)
             if world > 1:
                 from .parallel import all_reduce_sum
 
@@ -612,7 +629,6 @@ class StepEngine:
             recons = recon
         return pre_actvs, features, recon, recons
 
-    @torch.no_grad()
     def encode_layer(self, acts_norm: torch.Tensor, layer: int) -> torch.Tensor:
         """``Encoder.forward_layer`` (reference clt.py:134-145): ``acts_norm [..., D] @ W[layer] + b[layer]``
         on the contraction kernel, fp32 ``[..., F]`` out."""
@@ -636,7 +652,6 @@ class StepEngine:
         self._call("clt_export_blf", z, enc.b.data[layer:layer + 1] if enc.bias else None, out, B, 1, F, int(bf16), s)
         return out.reshape(*lead, F)
 
-    @torch.no_grad()
     def decode_layer(self, features: torch.Tensor, layer: int) -> torch.Tensor:
         """``Decoder.forward_layer`` / ``CrosslayerDecoder.forward_layer`` (reference clt.py:216-231, 304-317):
         the reconstruction of target ``layer`` from ``features [..., F]`` (per-layer decoder; a 4-D input
@@ -1225,12 +1240,16 @@ class StepEngine:
         i = st["step"]
         st["step"] = i + 1
         slot = i & 1
-        cmax_t = cnt.max() if cnt is not None else soon_dead.new_zeros(())
-        if i < 2:
-            exchange = cnt is not None and int(cmax_t) > k_aux   # blocking: first two steps only
+        if cnt is None:
+            exchange = False
+            st["host"][slot, 0].copy_(soon_dead.max(), non_blocking=True)
         else:
-            exchange = cnt is not None and 4 * int(st["host"][slot, 1]) > 3 * k_aux
-        st["host"][slot].copy_(torch.stack([soon_dead.max(), cmax_t]).to(torch.int32), non_blocking=True)
+            cmax_t = cnt.max()
+            if i < 2:
+                exchange = int(cmax_t) > k_aux                   # blocking: first two steps only
+            else:
+                exchange = 4 * int(st["host"][slot, 1]) > 3 * k_aux
+            st["host"][slot].copy_(torch.stack([soon_dead.max(), cmax_t]).to(torch.int32), non_blocking=True)
         st["evt"][slot].record()
         return exchange
 

@@ -141,7 +141,7 @@ class CrosslayerDecoder(_Layered):
             self.b.zero_()
 
     def blocks(self):
-        return [self.get_parameter(f"W_{t}") for t in range(self.n_layers)]
+        return [self._parameters[f"W_{t}"] for t in range(self.n_layers)]
 
     @torch.no_grad()
     def forward_layer(self, features, layer: int):

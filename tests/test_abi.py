@@ -96,3 +96,43 @@ def test_bench_work_model_names_are_entry_points():
         for k, v in work.items():
             assert k.split("[")[0] in protos, k
             assert v[0] in ("tensor", "hbm") and v[1] > 0, (name, k, v)
+
+
+def test_native_call_path_converts_like_ctypes():
+    """The compiled wrappers pass None, addresses, tensors, integers (masked like C) and floats as ctypes does, reject
+    what they cannot convert before calling, and leave ctypes' own pointer objects to ctypes."""
+    import pytest
+    import torch
+
+    L = _lib.lib()
+    assert set(L._native) == {n for n, (r, a) in L.protos.items() if r is ctypes.c_int and a}
+    name, types = "clt_adam_step", [t for _, t in L.protos["clt_adam_step"][1]]
+    seen = []
+
+    @ctypes.CFUNCTYPE(ctypes.c_int, *types)
+    def probe(*args):
+        seen.append(args)
+        return 7
+
+    t = torch.zeros(4)
+    values = {ctypes.c_void_p: [t, None, 4096, torch.nn.Parameter(t)], ctypes.c_int: [3, -1, True, 2 ** 40 + 5],
+              ctypes.c_int64: [2 ** 40, -2], ctypes.c_float: [0.1, 2]}
+    args = [values[ty][i % len(values[ty])] for i, ty in enumerate(types)]
+    mod = __import__("sys").modules[type(L).__module__]
+    loaded = L._native[name].__self__
+    try:
+        assert loaded.bind(name, ctypes.cast(probe, ctypes.c_void_p).value)
+        assert L._native[name](*args) == 7
+        assert probe(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]) == 7
+        assert seen[0] == seen[1]
+        for bad in (args[:-1], [object()] + args[1:], ["x"] * len(args)):
+            with pytest.raises(TypeError):
+                L._native[name](*bad)
+        assert len(seen) == 2
+    finally:
+        loaded.bind(name, ctypes.cast(L._fn[name], ctypes.c_void_p).value)
+    with pytest.raises(mod.CltError, match="bad dims"):
+        L.call("clt_encoder_fwd_store", None, None, None, 0, 1, 1, 1, 0, None, None)
+    dev = ctypes.c_void_p()
+    with pytest.raises((mod.CltError, ctypes.ArgumentError)):
+        L.call("clt_host_register", 0, 0, ctypes.byref(dev))
