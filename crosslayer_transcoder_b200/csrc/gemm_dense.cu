@@ -46,12 +46,14 @@ SimtOperands simt_operands(const Operand& a, const Operand& b) {
   return s;
 }
 
-template <class EpiF32, class EpiBf16>
+// A_MN / B_MN: the operand is MN-major (k_contig == 0), fixed by the op and so by the instantiation
+template <class EpiF32, class EpiBf16, bool A_MN, bool B_MN>
 int run_gemm(const GemmGeom& g, const Operand& a, const Operand& b, const typename EpiF32::Params& p32,
              const typename EpiBf16::Params& p16, int bf16, int* status, cudaStream_t stream) {
   if (bf16) {
     CLT_CHECK_ARG(status != nullptr, "the tensor-core path needs a device status word");
-    return tc::launch_gemm_tc<EpiBf16>(g, tc_operand(a), tc_operand(b), p16, status, device_sm_count(), stream);
+    CLT_CHECK_ARG(a.k_contig == (A_MN ? 0 : 1) && b.k_contig == (B_MN ? 0 : 1), "gemm: operand layout");
+    return tc::launch_gemm_tc<EpiBf16, A_MN, B_MN>(g, tc_operand(a), tc_operand(b), p16, status, device_sm_count(), stream);
   }
   return launch_gemm_simt<EpiF32>(g, simt_operands(a, b), p32, device_sm_count(), stream);
 }
@@ -107,7 +109,7 @@ int clt_encoder_fwd_act(const void* xn, const void* W_enc, const float* b_enc, c
                                       c_sparsity, use_tanh, want_pre};
   epi::EncJumpReLU<bf16_t>::Params p16{b_enc, theta, dec_norm, (bf16_t*)z_out, (bf16_t*)feat_out, fired_bits,
                                        loss_acc, c_sparsity, use_tanh, want_pre};
-  return run_gemm<epi::EncJumpReLU<float>, epi::EncJumpReLU<bf16_t>>(g, a, b, p32, p16, bf16, status,
+  return run_gemm<epi::EncJumpReLU<float>, epi::EncJumpReLU<bf16_t>, false, true>(g, a, b, p32, p16, bf16, status,
                                                                       (cudaStream_t)stream);
 }
 
@@ -119,7 +121,7 @@ int clt_encoder_fwd_store(const void* xn, const void* W_enc, void* z_out, int B,
   Operand a{xn, 1, B, D, L}, b{W_enc, 0, F, D, L};
   epi::StoreZ<float>::Params p32{(float*)z_out};
   epi::StoreZ<bf16_t>::Params p16{(bf16_t*)z_out};
-  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>>(g, a, b, p32, p16, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, true>(g, a, b, p32, p16, bf16, status, (cudaStream_t)stream);
 }
 
 int clt_decoder_dense_fwd(const void* feat, const void* W_dec, const float* b_dec, float* recon, int B, int L, int D,
@@ -149,7 +151,7 @@ int clt_decoder_dense_fwd_ws(const void* feat, const void* W_dec, const float* b
       if (parts * B * D <= ws_floats && parts <= 65535) {
         g.nz = (int)parts;
         epi::DecOut::Params pp{ws, nullptr, (long long)D, (long long)B * D};
-        if (int rc = run_gemm<epi::DecOut, epi::DecOut>(g, a, b, pp, pp, bf16, status, (cudaStream_t)stream)) return rc;
+        if (int rc = run_gemm<epi::DecOut, epi::DecOut, false, true>(g, a, b, pp, pp, bf16, status, (cudaStream_t)stream)) return rc;
         const long long slab = (long long)B * D;
         if (D % 4 == 0 && ((uintptr_t)recon | (uintptr_t)b_dec) % 16 == 0) {
           sum_parts_kernel<4><<<dim3((unsigned)((slab / 4 + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
@@ -164,7 +166,7 @@ int clt_decoder_dense_fwd_ws(const void* feat, const void* W_dec, const float* b
       g.kb_per_part = 0;  // the workspace is too small: whole chains
     }
   }
-  return run_gemm<epi::DecOut, epi::DecOut>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::DecOut, epi::DecOut, false, true>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
 }
 
 int clt_decoder_dense_fwd_push(const void* feat, const void* W_dec, const float* b_dec, const uint64_t* rank_bases,
@@ -188,7 +190,7 @@ int clt_decoder_dense_fwd_push(const void* feat, const void* W_dec, const float*
   p.zstride = (long long)D;
   p.slot_offset = (long long)my_slot * rows_per_rank * L * D;
   p.slot_bf16 = slot_bf16 ? 1 : 0;
-  return run_gemm<epi::DecOutPush, epi::DecOutPush>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::DecOutPush, epi::DecOutPush, false, true>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
 }
 
 int clt_decoder_dense_bwd_dfeat(const void* drecon, const void* W_dec, const void* z_in, const float* b_enc,
@@ -207,7 +209,7 @@ int clt_decoder_dense_bwd_dfeat(const void* drecon, const void* W_dec, const voi
                                         dnorm, bandwidth, lam, c_sparsity, pal, use_tanh, gscale};
   epi::DFeatJumpReLU<bf16_t>::Params p16{(const bf16_t*)z_in, b_enc, theta, dec_norm, (bf16_t*)dpre_out, dtheta, dbenc,
                                          dnorm, bandwidth, lam, c_sparsity, pal, use_tanh, gscale};
-  return run_gemm<epi::DFeatJumpReLU<float>, epi::DFeatJumpReLU<bf16_t>>(g, a, b, p32, p16, bf16, status,
+  return run_gemm<epi::DFeatJumpReLU<float>, epi::DFeatJumpReLU<bf16_t>, false, false>(g, a, b, p32, p16, bf16, status,
                                                                           (cudaStream_t)stream);
 }
 
@@ -220,7 +222,7 @@ int clt_decoder_dense_bwd_dfeat_raw(const void* drecon, const void* W_dec, void*
   Operand a{drecon, 1, B, D, L}, b{W_dec, 1, F, D, P};
   epi::StoreZ<float>::Params p32{(float*)g_out};
   epi::StoreZ<bf16_t>::Params p16{(bf16_t*)g_out};
-  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>>(g, a, b, p32, p16, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, false>(g, a, b, p32, p16, bf16, status, (cudaStream_t)stream);
 }
 
 int clt_decoder_dense_bwd_dw(const void* feat, const void* drecon, float* dW, const float* rowcoef,
@@ -234,7 +236,7 @@ int clt_decoder_dense_bwd_dw(const void* feat, const void* drecon, float* dW, co
   // A: feat[s]^T, stored [B (K), F (M)] with M contiguous; B: drecon[t], stored [B (K), D (N)] with N contiguous
   Operand a{feat, 0, F, B, L}, b{drecon, 0, D, B, L};
   epi::GradOut::Params p{dW, rowcoef, W_master, crosslayer ? 1 : 0};
-  return run_gemm<epi::GradOut, epi::GradOut>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::GradOut, epi::GradOut, true, true>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
 }
 
 int clt_encoder_dense_bwd_dw(const void* xn, const void* dpre, float* dW, int B, int L, int D, int F, int bf16,
@@ -244,7 +246,7 @@ int clt_encoder_dense_bwd_dw(const void* xn, const void* dpre, float* dW, int B,
   GemmGeom g{kBatched, D, F, B, L, L};
   Operand a{xn, 0, D, B, L}, b{dpre, 0, F, B, L};
   epi::GradOut::Params p{dW, nullptr, nullptr, 0};
-  return run_gemm<epi::GradOut, epi::GradOut>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::GradOut, epi::GradOut, true, true>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
 }
 
 }  // extern "C"

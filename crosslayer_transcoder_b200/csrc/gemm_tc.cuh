@@ -586,21 +586,10 @@ int launch_gemm_tc_tile(const GemmGeom& g, const TcOperand& a, const TcOperand& 
 }
 
 template <class Epi, bool A_MN, bool B_MN>
-int launch_gemm_tc_impl(const GemmGeom& g, const TcOperand& a, const TcOperand& b, const typename Epi::Params& ep,
-                        int* status, int num_sms, cudaStream_t stream) {
-  if (use_pair(g, num_sms)) return launch_gemm_tc_tile<Epi, A_MN, B_MN, true>(g, a, b, ep, status, num_sms, stream);
-  return launch_gemm_tc_tile<Epi, A_MN, B_MN, false>(g, a, b, ep, status, num_sms, stream);
-}
-
-template <class Epi>
 int launch_gemm_tc(const GemmGeom& g, const TcOperand& a, const TcOperand& b, const typename Epi::Params& ep,
                    int* status, int num_sms, cudaStream_t stream) {
-  if (a.mn_major) {
-    if (b.mn_major) return launch_gemm_tc_impl<Epi, true, true>(g, a, b, ep, status, num_sms, stream);
-    return launch_gemm_tc_impl<Epi, true, false>(g, a, b, ep, status, num_sms, stream);
-  }
-  if (b.mn_major) return launch_gemm_tc_impl<Epi, false, true>(g, a, b, ep, status, num_sms, stream);
-  return launch_gemm_tc_impl<Epi, false, false>(g, a, b, ep, status, num_sms, stream);
+  if (use_pair(g, num_sms)) return launch_gemm_tc_tile<Epi, A_MN, B_MN, true>(g, a, b, ep, status, num_sms, stream);
+  return launch_gemm_tc_tile<Epi, A_MN, B_MN, false>(g, a, b, ep, status, num_sms, stream);
 }
 
 }  // namespace tc
