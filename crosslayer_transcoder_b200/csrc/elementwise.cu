@@ -622,7 +622,34 @@ int loss_bwd(const float* recon, const float* aux, const void* batch, int in_dty
 //           loss_acc[1] += sum tanh(feat n c) (or the product);  fired bits
 // backward: dpre, dtheta, db_enc, d dec_norm from g = dL/dfeat exactly as csrc/epilogues.cuh states
 // ---------------------------------------------------------------------------------
-constexpr int kActRows = 4;
+template <class T>
+constexpr int kActRows = sizeof(T) == 2 ? 4 : 2;  // the same bytes in flight
+
+// tanh of 8 values.  tanhf branches for every value, which keeps the eight from overlapping and made the sweeps with a
+// sparsity penalty issue-bound.  Here one branch covers all eight: below 0.7 (where penalties live: feature x decoder norm x c)
+// tanh(x) = x + x^3 P(x^2), P of degree 5 fitted by iteratively reweighted least squares to the smallest largest
+// relative error (7e-10; in fp32 0.74 ulp against float64, tanhf is specified to 2); anything larger takes tanhf.
+// 12 x 4000 x 10000 bf16 with penalty: forward 745 -> 660 us, backward 1370 -> 1210 us.
+__device__ __forceinline__ void tanh8(float (&v)[8]) {
+  float top = 0.f, t[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float s = v[q] * v[q];
+    top = fmaxf(top, s);
+    float p = fmaf(s, 0.001895663677714765f, -0.007883304730057716f);
+    p = fmaf(s, p, 0.02157105877995491f);
+    p = fmaf(s, p, -0.05392095446586609f);
+    p = fmaf(s, p, 0.133329838514328f);
+    p = fmaf(s, p, -0.33333325386047363f);
+    t[q] = fmaf(p, v[q] * s, v[q]);
+  }
+  if (top > 0.49f) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q] = tanhf(v[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = t[q];
+}
 
 template <class T>
 __global__ void __launch_bounds__(128)
@@ -648,7 +675,7 @@ act_fwd_kernel(const T* __restrict__ z, const float* __restrict__ b_enc, const f
     }
     unsigned mask = 0u;
     auto row = [&](const Raw8<T>& zr, size_t o) {
-      float fv[8];
+      float fv[8], wv[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const float pre = zr.get(q) + bb[q];
@@ -656,21 +683,23 @@ act_fwd_kernel(const T* __restrict__ z, const float* __restrict__ b_enc, const f
         fv[q] = f;
         mask |= (f > 0.f) ? (1u << q) : 0u;
         if (want_pre) s_pre += fmaxf(-pre, 0.f);
-        if (sp) {
-          const float w = f * nn[q];
-          s_sp += use_tanh ? tanhf(w) : w;
-        }
+        wv[q] = f * nn[q];
+      }
+      if (sp) {
+        if (use_tanh) tanh8(wv);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s_sp += wv[q];
       }
       store8<T>(feat + o, fv);
     };
     size_t o = ((size_t)l * B + r0) * F + f0;
     int r = r0;
-    for (; r + kActRows <= r1; r += kActRows) {
-      Raw8<T> zr[kActRows];
+    for (; r + kActRows<T> <= r1; r += kActRows<T>) {
+      Raw8<T> zr[kActRows<T>];
 #pragma unroll
-      for (int i = 0; i < kActRows; ++i) zr[i].load(z + o + (size_t)i * F);
+      for (int i = 0; i < kActRows<T>; ++i) zr[i].load(z + o + (size_t)i * F);
 #pragma unroll
-      for (int i = 0; i < kActRows; ++i, o += F) row(zr[i], o);
+      for (int i = 0; i < kActRows<T>; ++i, o += F) row(zr[i], o);
     }
     for (; r < r1; ++r, o += F) {
       Raw8<T> zr;
@@ -723,7 +752,15 @@ act_bwd_kernel(const T* g, const T* __restrict__ z, const float* __restrict__ b_
 #pragma unroll
   for (int q = 0; q < 8; ++q) sb[q] = 0.f, st[q] = 0.f, sn[q] = 0.f;
   auto row = [&](const Raw8<T>& gr, const Raw8<T>& zr, size_t o) {
-    float dp[8];
+    float dp[8], tw[8];
+    if (sp && use_tanh) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float pre = zr.get(q) + bb[q];
+        tw[q] = (pre > tt[q] && pre > 0.f) ? pre * nn[q] : 0.f;
+      }
+      tanh8(tw);
+    }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const float th = tt[q];
@@ -731,11 +768,7 @@ act_bwd_kernel(const T* g, const T* __restrict__ z, const float* __restrict__ b_
       float gs = gr.get(q);
       if (sp) {
         const float f = (pre > th && pre > 0.f) ? pre : 0.f;
-        float d1 = 1.f;
-        if (use_tanh) {
-          const float tw = tanhf(f * nn[q]);
-          d1 = 1.f - tw * tw;
-        }
+        const float d1 = use_tanh ? 1.f - tw[q] * tw[q] : 1.f;
         gs = fmaf(lam * d1, nn[q], gs);
         sn[q] = fmaf(lam * d1 * c_sparsity, f, sn[q]);
       }
@@ -752,12 +785,12 @@ act_bwd_kernel(const T* g, const T* __restrict__ z, const float* __restrict__ b_
   // g and dpre may be one buffer: a thread writes only elements that it has read
   size_t o = ((size_t)l * B + r0) * F + f0;
   int r = r0;
-  for (; r + kActRows <= r1; r += kActRows) {
-    Raw8<T> gr[kActRows], zr[kActRows];
+  for (; r + kActRows<T> <= r1; r += kActRows<T>) {
+    Raw8<T> gr[kActRows<T>], zr[kActRows<T>];
 #pragma unroll
-    for (int i = 0; i < kActRows; ++i) gr[i].load(g + o + (size_t)i * F), zr[i].load(z + o + (size_t)i * F);
+    for (int i = 0; i < kActRows<T>; ++i) gr[i].load(g + o + (size_t)i * F), zr[i].load(z + o + (size_t)i * F);
 #pragma unroll
-    for (int i = 0; i < kActRows; ++i, o += F) row(gr[i], zr[i], o);
+    for (int i = 0; i < kActRows<T>; ++i, o += F) row(gr[i], zr[i], o);
   }
   for (; r < r1; ++r, o += F) {
     Raw8<T> gr, zr;
