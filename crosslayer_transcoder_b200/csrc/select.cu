@@ -437,7 +437,7 @@ select_topk_warp_kernel(const T* __restrict__ z, const float* __restrict__ b_enc
 // candidate list in shared memory.
 //
 //   * A value joins the list when its key is at least tau (tau starts at the smallest positive key).
-//   * When the list could overflow, the warp finds the k-th largest key T of the list (bisection on the
+//   * When the list has grown enough (trim_at), the warp finds the k-th largest key T of the list (bisection on the
 //     key bits over values held in registers), keeps the k best entries and raises tau to T + 1: from
 //     then on only values that would displace one of the k held ones join (a value equal to the current
 //     k-th is interchangeable with it).  After the first few hundred elements tau sits near the row's
@@ -485,9 +485,9 @@ struct ChunkLoader<float> {
 
 // Keep the k best of the n entries of a warp's candidate list (n <= kStreamCap, n > k); returns the k-th
 // largest key.  Entries equal to it are kept in list order until k are held.
-__device__ __forceinline__ unsigned stream_keep_top(float* cv, int* ci, int n, int k) {
+template <int kPer>
+__device__ __forceinline__ unsigned stream_keep_top_n(float* cv, int* ci, int n, int k) {
   const int lane = threadIdx.x & 31;
-  constexpr int kPer = kStreamCap / 32;
   unsigned key[kPer];
 #pragma unroll
   for (int q = 0; q < kPer; ++q) key[q] = (lane + 32 * q) < n ? __float_as_uint(cv[lane + 32 * q]) : 0u;
@@ -527,6 +527,13 @@ __device__ __forceinline__ unsigned stream_keep_top(float* cv, int* ci, int n, i
   return Tk;
 }
 
+// the registers that a list of n entries needs, and no more, take part in the bisection's 31 counts
+__device__ __forceinline__ unsigned stream_keep_top(float* cv, int* ci, int n, int k) {
+  if (n <= 128) return stream_keep_top_n<4>(cv, ci, n, k);
+  if (n <= 256) return stream_keep_top_n<8>(cv, ci, n, k);
+  return stream_keep_top_n<kStreamCap / 32>(cv, ci, n, k);
+}
+
 template <class T>
 __global__ void __launch_bounds__(kStreamWarps * 32, 4)
 select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_enc, int* __restrict__ idx_out,
@@ -547,6 +554,11 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
   int* cnt = &c_cnt[warp];
   if (lane == 0) *cnt = 0;
   __syncwarp();
+  // Trim when 64 (or k) entries have joined the k that are held, and before the next step could overflow the list: a
+  // stale tau lets 4 values of a step join in the middle of a row of 32768, which costs more than a trim of 128
+  // (12 x 4000 rows of 32768, k = 32: 1.39 -> 1.15 ms; 12 x 2047 of 20000, k = 16: 0.51 -> 0.38 ms; trimming only when the list
+  // was full, always over 512 registers, before).
+  const int trim_at = min(kStreamCap - 256, k + max(64, k));
   using CL = ChunkLoader<T>;
   // 256 columns per step (8 per lane); the next step's row values are requested before this step's are used
   const int n_steps = F / 256;              // whole steps; the ragged end (F % 256, a multiple of 8) follows
@@ -584,7 +596,7 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
     }
     __syncwarp();
     const int count = *reinterpret_cast<volatile int*>(cnt);
-    if (count > kStreamCap - 256) {        // the next step could overflow the list: keep the k best, raise tau
+    if (count > trim_at) {                 // keep the k best, raise tau
       if (count > k) {
         tau = __uint_as_float(stream_keep_top(cv, ci, count, k) + 1u);
         if (lane == 0) *cnt = k;
