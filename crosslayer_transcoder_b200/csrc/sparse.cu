@@ -115,6 +115,9 @@ sparse_dec_fwd_kernel(const int* __restrict__ idx, const float* __restrict__ val
                       const float* __restrict__ b_dec, float* __restrict__ recon, int B, int L, int D, int F, int k,
                       int crosslayer, int* status, PushDst push) {
   extern __shared__ float red[];  // [4][D]
+  // rows in flight per warp; wider rows fill the registers alone (1000 tokens x 12 layers x 16 entries of 768 bf16
+  // columns: 310 -> 245 us against one row)
+  constexpr int kRows = VPL * sizeof(T) <= 8 ? 2 : 1;
   const int b = blockIdx.x, t = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = D / 8;
@@ -133,23 +136,33 @@ sparse_dec_fwd_kernel(const int* __restrict__ idx, const float* __restrict__ val
       e0 = (size_t)s * npl + __ldg(row_start + (size_t)s * B + b);
       n = __ldg(row_cnt + (size_t)s * B + b);
     }
-    for (int j = warp; j < n; j += 4) {
-      const float v = __ldg(val + e0 + j);
-      if (v == 0.f) break;  // valid slots come first
-      const int f = __ldg(idx + e0 + j);
-      if (f < 0 || f >= F) {
-        report_status(status, kBadIndex);
-        continue;
+    for (int j0 = warp; j0 < n; j0 += 4 * kRows) {
+      float v[kRows];
+      typename Vec8<T>::Raw x[kRows][VPL];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const int j = j0 + 4 * r;
+        v[r] = j < n ? __ldg(val + e0 + j) : 0.f;
+        int f = j < n ? __ldg(idx + e0 + j) : 0;
+        if (v[r] != 0.f && (f < 0 || f >= F)) {
+          report_status(status, kBadIndex);
+          v[r] = 0.f;
+        }
+        const T* row = W + (p * F + (v[r] != 0.f ? f : 0)) * D;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+          const int c = lane + 32 * i;
+          x[r][i] = (v[r] != 0.f && c < nvec) ? Vec8<T>::load_raw(row + 8 * c) : Vec8<T>::zero();
+        }
       }
-      const T* row = W + (p * F + f) * D;
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int c = lane + 32 * i;
-        if (c < nvec) {
+      for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
           float w[8];
-          Vec8<T>::load(row + 8 * c, w);
+          Vec8<T>::unpack(x[r][i], w);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc[i][q] = fmaf(v, w[q], acc[i][q]);
+          for (int q = 0; q < 8; ++q) acc[i][q] = fmaf(v[r], w[q], acc[i][q]);
         }
       }
     }
