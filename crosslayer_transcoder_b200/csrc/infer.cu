@@ -9,7 +9,7 @@
 namespace clt {
 namespace {
 
-// Rows of V consecutive elements in registers; V = 8 needs rows that start on 16-byte boundaries.
+// Rows of V consecutive elements in registers; V = 8 needs rows that start on 32-byte boundaries.
 template <class T, int V>
 __device__ __forceinline__ void load_row(const T* p, float (&o)[V]) {
   if constexpr (V == 1) {
@@ -26,11 +26,8 @@ __device__ __forceinline__ void load_row(const T* p, float (&o)[V]) {
       o[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
     }
   } else {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const float4 t = __ldcs(reinterpret_cast<const float4*>(p) + j);
-      o[4 * j] = t.x, o[4 * j + 1] = t.y, o[4 * j + 2] = t.z, o[4 * j + 3] = t.w;
-    }
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(p)), b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+    o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
   }
 }
 template <class T, int V>
@@ -44,9 +41,7 @@ __device__ __forceinline__ void store_row(T* p, const float (&v)[V]) {
     *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
                                               pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
   } else {
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      reinterpret_cast<float4*>(p)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    st_f32x8(p, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
   }
 }
 template <class T>
@@ -56,8 +51,8 @@ __device__ __forceinline__ float rounded(float x) {
 
 // The three layout kernels below are bound by HBM.  A CTA covers 256 V columns of one layer (blockIdx.x, blockIdx.z) and
 // walks batch rows (blockIdx.y strided), so an element costs no division and the per-column parameters stay in
-// registers; V = 8 makes every access 16 bytes wide.  export at [12, 1000, 10000] bf16: 472 -> 162 us (4.4 TB/s), one
-// element per thread and step with two 64-bit divisions before; act_export at [12, 333, 24576] 228 us (5.2 TB/s) for what
+// registers; V = 8 makes every load 16 and every fp32 store 32 bytes wide.  export at [12, 1000, 10000] bf16: 472 -> 128 us (5.6 TB/s; 162 us with two 16-byte stores), one
+// element per thread and step with two 64-bit divisions before; act_export at [12, 333, 24576] 195 us (6.0 TB/s) for what
 // an activation sweep and two exports took 900 us.
 
 // out[b, l, f] = src[l, b, f] (+ bias[l, f])     layer-major T -> token-major fp32
@@ -141,12 +136,9 @@ inline dim3 row_grid(int B, int L, long long F, int V) {
   if (gy > B) gy = B;
   return dim3((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535), (unsigned)L);
 }
-inline bool aligned16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
-  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d) & 15) == 0;
-}
 template <class T>
 int launch_import(const float* src, long long ld, void* dst, int B, int L, long long F, cudaStream_t s) {
-  if (F % 8 == 0 && ld % 4 == 0 && aligned16(src, dst))
+  if (F % 8 == 0 && ld % 8 == 0 && aligned32(src) && aligned32(dst))
     import_rows_kernel<T, 8><<<row_grid(B, L, F, 8), 256, 0, s>>>(src, ld, (T*)dst, B, F);
   else
     import_rows_kernel<T, 1><<<row_grid(B, L, F, 1), 256, 0, s>>>(src, ld, (T*)dst, B, F);
@@ -155,7 +147,7 @@ int launch_import(const float* src, long long ld, void* dst, int B, int L, long 
 }
 template <class T>
 int launch_export(const void* src, const float* bias, float* out, int B, int L, long long F, cudaStream_t s) {
-  if (F % 8 == 0 && aligned16(src, out))
+  if (F % 8 == 0 && aligned32(src) && aligned32(out))
     export_blf_kernel<T, 8><<<row_grid(B, L, F, 8), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
   else
     export_blf_kernel<T, 1><<<row_grid(B, L, F, 1), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
@@ -224,7 +216,8 @@ int clt_act_export(const void* z, const float* bias, const float* theta, float* 
   CLT_CHECK_ARG(z && bias && pre && feat && features && B > 0 && L > 0 && L <= 65535 && F > 0,
                 "act_export: bad arguments");
   CLT_CHECK_ARG(F % 8 == 0, "act_export: d_features=%lld must be a multiple of 8", (long long)F);
-  CLT_CHECK_ARG(aligned16(z, pre, feat, features), "act_export: buffers must be 16-byte aligned");
+  CLT_CHECK_ARG(aligned32(z) && aligned32(pre) && aligned32(feat) && aligned32(features),
+                "act_export: buffers must be 32-byte aligned");
   const dim3 grid = row_grid(B, L, F, 8);
   cudaStream_t s = (cudaStream_t)stream;
   if (bf16)

@@ -491,9 +491,8 @@ sparse_bwd_dec_kernel(const int* __restrict__ col_ptr, const int* __restrict__ e
   for (int i = 0; i < VPL; ++i) {
     const int c = lane + 32 * i;
     if (c < nvec) {
-      float4* o = reinterpret_cast<float4*>(dW + roff + 8 * c);
-      __stcs(o, make_float4(g[i][0], g[i][1], g[i][2], g[i][3]));
-      __stcs(o + 1, make_float4(g[i][4], g[i][5], g[i][6], g[i][7]));
+      st_cs8(dW + roff + 8 * c, make_float4(g[i][0], g[i][1], g[i][2], g[i][3]),
+             make_float4(g[i][4], g[i][5], g[i][6], g[i][7]));
     }
   }
 }
@@ -533,9 +532,8 @@ sparse_bwd_dec_group_kernel(const int* __restrict__ col_ptr, const int* __restri
       for (int i = 0; i < VPL; ++i) {
         const int c = lane + 32 * i;
         if (c < nvec) {
-          float4* o = reinterpret_cast<float4*>(dW + row0 + (size_t)j * D + 8 * c);
-          __stcs(o, make_float4(0.f, 0.f, 0.f, 0.f));
-          __stcs(o + 1, make_float4(0.f, 0.f, 0.f, 0.f));
+          const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+          st_cs8(dW + row0 + (size_t)j * D + 8 * c, zero, zero);
         }
       }
     }
@@ -629,9 +627,8 @@ sparse_bwd_dec_group_kernel(const int* __restrict__ col_ptr, const int* __restri
     for (int i = 0; i < VPL; ++i) {
       const int c = lane + 32 * i;
       if (c < nvec) {
-        float4* o = reinterpret_cast<float4*>(dW + row0 + (size_t)fi * D + 8 * c);
-        __stcs(o, make_float4(g[i][0], g[i][1], g[i][2], g[i][3]));
-        __stcs(o + 1, make_float4(g[i][4], g[i][5], g[i][6], g[i][7]));
+        st_cs8(dW + row0 + (size_t)fi * D + 8 * c, make_float4(g[i][0], g[i][1], g[i][2], g[i][3]),
+               make_float4(g[i][4], g[i][5], g[i][6], g[i][7]));
       }
     }
     if (!has_next) break;
@@ -839,8 +836,8 @@ sparse_bwd_enc_vec_kernel(const int* __restrict__ col_ptr, const int* __restrict
     for (int i = 0; i < 8; ++i) {
       float* o = dW + ((size_t)l * D + d + i) * F + f0;
       if (vec) {
-        __stcs(reinterpret_cast<float4*>(o), make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]));
-        __stcs(reinterpret_cast<float4*>(o) + 1, make_float4(acc[4][i], acc[5][i], acc[6][i], acc[7][i]));
+        st_cs8(o, make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]),
+               make_float4(acc[4][i], acc[5][i], acc[6][i], acc[7][i]));
       } else {
 #pragma unroll
         for (int q = 0; q < kEncFB; ++q)
