@@ -27,7 +27,8 @@ def test_streaming_activation(L, B, F, scale, bf16):
     f32 = torch.where((pre > theta[:, None]) & (pre > 0), pre, torch.zeros_like(pre))
     assert torch.equal(feat, f32.to(T))
     bits = (f32 > 0).any(dim=1)
-    got = torch.stack([(fired[:, i // 32] >> (i % 32)) & 1 for i in range(F)], dim=1).bool()
+    f = torch.arange(F, device=dev)
+    got = ((fired[:, f // 32] >> (f % 32)) & 1).bool()
     assert torch.equal(got, bits)
     f, n = f32.double(), norm.double()[:, None] * c
     tw = torch.tanh(f * n)
