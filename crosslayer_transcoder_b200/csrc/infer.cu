@@ -51,9 +51,9 @@ __device__ __forceinline__ float rounded(float x) {
 
 // The three layout kernels below are bound by HBM.  A CTA covers 256 V columns of one layer (blockIdx.x, blockIdx.z) and
 // walks batch rows (blockIdx.y strided), so an element costs no division and the per-column parameters stay in
-// registers; V = 8 makes every load 16 and every fp32 store 32 bytes wide.  export at [12, 1000, 10000] bf16: 472 -> 128 us (5.6 TB/s; 162 us with two 16-byte stores), one
-// element per thread and step with two 64-bit divisions before; act_export at [12, 333, 24576] 195 us (6.0 TB/s) for what
-// an activation sweep and two exports took 900 us.
+// registers; V = 8 makes every load 16 and every fp32 store 32 bytes wide.  export at [12, 1000, 10000] bf16:
+// 472 -> 128 us (5.6 TB/s; 162 us with two 16-byte stores), one element per thread and step with two 64-bit divisions
+// before; act_export at [12, 333, 24576] 195 us (6.0 TB/s) for what an activation sweep and two exports took 900 us.
 
 // out[b, l, f] = src[l, b, f] (+ bias[l, f])     layer-major T -> token-major fp32
 template <class T, int V>
