@@ -12,6 +12,7 @@ import hashlib
 import importlib.machinery
 import importlib.util
 import re
+import sysconfig
 from pathlib import Path
 from typing import Dict, List, Tuple
 
@@ -20,7 +21,8 @@ import torch
 PKG = Path(__file__).resolve().parent
 HEADER = PKG.parent / "include" / "clt_b200.h"
 LIB_PATH = PKG / "libclt_b200.so"
-BINDING_PATH = PKG / "_clt_call.so"
+#: The name carries the interpreter's ABI tag: a tree built under one Python and imported under another has none.
+BINDING_PATH = PKG / ("_clt_call" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 _CTYPES = {
     "int": ctypes.c_int,
@@ -77,14 +79,17 @@ class _Lib:
         self._device_ok = set()
 
     def _bind_native(self):
-        """{name: wrapper} of the compiled call path (``build.binding_source``), empty where it was not built or was built
-        for other prototypes."""
+        """{name: wrapper} of the compiled call path (``build.binding_source``), empty where it was not built, does not
+        load, or was built for other prototypes: calls then go through ctypes."""
         if not BINDING_PATH.exists():
             return {}
         loader = importlib.machinery.ExtensionFileLoader("_clt_call", str(BINDING_PATH))
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_clt_call", loader))
-        loader.exec_module(mod)
-        if mod.prototypes != prototypes_digest(self.protos):
+        try:
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_clt_call", loader))
+            loader.exec_module(mod)
+        except ImportError:
+            return {}
+        if getattr(mod, "prototypes", None) != prototypes_digest(self.protos):
             return {}
         return {n: getattr(mod, n) for n, fn in self._fn.items()
                 if hasattr(mod, n) and mod.bind(n, ctypes.cast(fn, ctypes.c_void_p).value)}

@@ -76,8 +76,8 @@ static int as_f32(PyObject* a, float* out) {
 
 
 def binding_source(protos) -> str:
-    """C source of the ``_clt_call`` extension module for ``_lib.parse_header``'s prototypes.  ``bind(name, address)`` gives
-    a wrapper its entry point; a wrapper raises TypeError before it calls anything."""
+    """C source of the ``_clt_call`` extension module for ``_lib.parse_header``'s prototypes.  ``bind(name, address)``
+    gives a wrapper its entry point; a wrapper raises TypeError before it calls anything."""
     from ._lib import prototypes_digest
 
     kinds = {ctypes.c_void_p: ("void*", "void*", "as_ptr"), ctypes.c_int: ("int", "int64_t", "as_i64"),
@@ -115,12 +115,18 @@ def binding_source(protos) -> str:
     return "\n".join(out)
 
 
+def _binding_tools():
+    """(folder of Python's headers, C compiler), None for what this host does not have."""
+    include = sysconfig.get_paths()["include"]
+    return include if (Path(include) / "Python.h").exists() else None, shutil.which("gcc") or shutil.which("cc")
+
+
 def build_binding(force: bool = False):
     """Compile the native call path.  Without Python's headers there is none, and calls go through ctypes."""
     from ._lib import BINDING_PATH, HEADER, parse_header
 
-    include, cc = sysconfig.get_paths()["include"], shutil.which("gcc") or shutil.which("cc")
-    if cc is None or not (Path(include) / "Python.h").exists():
+    include, cc = _binding_tools()
+    if include is None or cc is None:
         BINDING_PATH.unlink(missing_ok=True)
         return None
     if force or _stale(BINDING_PATH, [HEADER, Path(__file__)]):

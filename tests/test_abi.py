@@ -104,7 +104,11 @@ def test_native_call_path_converts_like_ctypes():
     import pytest
     import torch
 
+    from crosslayer_transcoder_b200 import build
+
     L = _lib.lib()
+    if not L._native and None in build._binding_tools():
+        pytest.skip("no Python headers or C compiler: calls go through ctypes")
     assert set(L._native) == {n for n, (r, a) in L.protos.items() if r is ctypes.c_int and a}
     name, types = "clt_adam_step", [t for _, t in L.protos["clt_adam_step"][1]]
     seen = []
@@ -136,3 +140,23 @@ def test_native_call_path_converts_like_ctypes():
     dev = ctypes.c_void_p()
     with pytest.raises((mod.CltError, ctypes.ArgumentError)):
         L.call("clt_host_register", 0, 0, ctypes.byref(dev))
+
+
+def test_call_path_that_cannot_load_leaves_ctypes(tmp_path, monkeypatch):
+    """An extension of another Python has another name; one that does not load, or is some other module, is passed over."""
+    import sysconfig
+
+    import pytest
+
+    # the suffix names this interpreter, so a tree that another one built has no such file
+    assert _lib.BINDING_PATH.name == "_clt_call" + sysconfig.get_config_var("EXT_SUFFIX")
+    for content in (b"", b"not an object file"):
+        path = tmp_path / "_clt_call.so"
+        path.write_bytes(content)
+        monkeypatch.setattr(_lib, "BINDING_PATH", path)
+        L = _lib._Lib()
+        assert L._native == {}
+        with pytest.raises(_lib.CltError, match="bad dims"):
+            L.call("clt_encoder_fwd_store", None, None, None, 0, 1, 1, 1, 0, None, None)
+    monkeypatch.setattr(_lib, "BINDING_PATH", tmp_path / "absent.so")
+    assert _lib._Lib()._native == {}
