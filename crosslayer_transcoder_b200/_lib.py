@@ -8,7 +8,6 @@ first use raises.
 from __future__ import annotations
 
 import ctypes
-import hashlib
 import importlib.machinery
 import importlib.util
 import re
@@ -52,11 +51,6 @@ def parse_header(path: Path = HEADER) -> Dict[str, Tuple[object, List[Tuple[str,
     return protos
 
 
-def prototypes_digest(protos) -> str:
-    text = repr([(n, r.__name__, [t.__name__ for _, t in args]) for n, (r, args) in protos.items()])
-    return hashlib.sha256(text.encode()).hexdigest()
-
-
 class CltError(RuntimeError):
     pass
 
@@ -80,7 +74,9 @@ class _Lib:
 
     def _bind_native(self):
         """{name: wrapper} of the compiled call path (``build.binding_source``), empty where it was not built, does not
-        load, or was built for other prototypes: calls then go through ctypes."""
+        load, or was built from other prototypes or conversions: calls then go through ctypes."""
+        from .build import binding_source
+
         if not BINDING_PATH.exists():
             return {}
         loader = importlib.machinery.ExtensionFileLoader("_clt_call", str(BINDING_PATH))
@@ -89,7 +85,7 @@ class _Lib:
             loader.exec_module(mod)
         except ImportError:
             return {}
-        if getattr(mod, "prototypes", None) != prototypes_digest(self.protos):
+        if getattr(mod, "source", None) != binding_source(self.protos)[0]:
             return {}
         return {n: getattr(mod, n) for n, fn in self._fn.items()
                 if hasattr(mod, n) and mod.bind(n, ctypes.cast(fn, ctypes.c_void_p).value)}

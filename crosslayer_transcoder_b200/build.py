@@ -3,6 +3,7 @@ in-tree with nvcc for sm_100a.  ``python -m crosslayer_transcoder_b200.build`` r
 from __future__ import annotations
 
 import ctypes
+import hashlib
 import os
 import shutil
 import subprocess
@@ -75,11 +76,10 @@ static int as_f32(PyObject* a, float* out) {
 """
 
 
-def binding_source(protos) -> str:
-    """C source of the ``_clt_call`` extension module for ``_lib.parse_header``'s prototypes.  ``bind(name, address)``
-    gives a wrapper its entry point; a wrapper raises TypeError before it calls anything."""
-    from ._lib import prototypes_digest
-
+def binding_source(protos):
+    """(digest, text): C source of the ``_clt_call`` extension module for ``_lib.parse_header``'s prototypes.  ``bind(name, address)``
+    gives a wrapper its entry point; a wrapper raises TypeError before it calls anything.  The module's
+    ``source`` is the digest, so that one which was made from another text is recognised."""
     kinds = {ctypes.c_void_p: ("void*", "void*", "as_ptr"), ctypes.c_int: ("int", "int64_t", "as_i64"),
              ctypes.c_int64: ("int64_t", "int64_t", "as_i64"), ctypes.c_float: ("float", "float", "as_f32")}
     names = [n for n, (ret, args) in protos.items() if ret is ctypes.c_int and args]
@@ -110,9 +110,11 @@ def binding_source(protos) -> str:
     out.append("  {0}};\nstatic struct PyModuleDef def = {PyModuleDef_HEAD_INIT, \"_clt_call\", 0, -1, methods};")
     out.append('PyMODINIT_FUNC PyInit__clt_call(void) {\n  s_data_ptr = PyUnicode_InternFromString("data_ptr");\n'
                '  PyObject* m = s_data_ptr ? PyModule_Create(&def) : 0;\n'
-               f'  if (m) PyModule_AddStringConstant(m, "prototypes", "{prototypes_digest(protos)}");\n'
+               '  if (m) PyModule_AddStringConstant(m, "source", SOURCE);\n'
                '  return m;\n}\n')
-    return "\n".join(out)
+    text = "\n".join(out)
+    digest = hashlib.sha256(text.encode()).hexdigest()
+    return digest, f'#define SOURCE "{digest}"\n{text}'
 
 
 def _binding_tools():
@@ -123,16 +125,16 @@ def _binding_tools():
 
 def build_binding(force: bool = False):
     """Compile the native call path.  Without Python's headers there is none, and calls go through ctypes."""
-    from ._lib import BINDING_PATH, HEADER, parse_header
+    from ._lib import BINDING_PATH, parse_header
 
     include, cc = _binding_tools()
     if include is None or cc is None:
         BINDING_PATH.unlink(missing_ok=True)
         return None
-    if force or _stale(BINDING_PATH, [HEADER, Path(__file__)]):
+    src, (_, text) = OBJ / "clt_call.c", binding_source(parse_header())
+    if force or not src.exists() or src.read_text() != text or _stale(BINDING_PATH, [src]):
         OBJ.mkdir(exist_ok=True)
-        src = OBJ / "clt_call.c"
-        src.write_text(binding_source(parse_header()))
+        src.write_text(text)
         cmd = [cc, "-O2", "-shared", "-fPIC", f"-I{include}", str(src), "-o", str(BINDING_PATH)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:

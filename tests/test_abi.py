@@ -160,3 +160,21 @@ def test_call_path_that_cannot_load_leaves_ctypes(tmp_path, monkeypatch):
             L.call("clt_encoder_fwd_store", None, None, None, 0, 1, 1, 1, 0, None, None)
     monkeypatch.setattr(_lib, "BINDING_PATH", tmp_path / "absent.so")
     assert _lib._Lib()._native == {}
+
+
+def test_call_path_of_another_source_is_passed_over(tmp_path, monkeypatch):
+    """A compiled call path is used only if it was made from today's conversions, not just from today's prototypes."""
+    import shutil
+
+    import pytest
+
+    from crosslayer_transcoder_b200 import build
+
+    if not _lib._Lib()._native:
+        pytest.skip("no Python headers or C compiler: calls go through ctypes")
+    path = tmp_path / _lib.BINDING_PATH.name
+    shutil.copy(_lib.BINDING_PATH, path)        # a copy: a module that was loaded from a file is loaded once
+    monkeypatch.setattr(_lib, "BINDING_PATH", path)
+    assert _lib._Lib()._native
+    monkeypatch.setattr(build, "_C_PRELUDE", build._C_PRELUDE + "/* converts otherwise */")
+    assert _lib._Lib()._native == {}
