@@ -49,9 +49,10 @@ __device__ __forceinline__ float rounded(float x) {
   return sizeof(T) == 2 ? bf16_round(x) : x;
 }
 
-// The three layout kernels below are bound by HBM.  A CTA covers 256 V columns of one layer (blockIdx.x, blockIdx.z) and
-// walks batch rows (blockIdx.y strided), so an element costs no division and the per-column parameters stay in
-// registers; V = 8 makes every load 16 and every fp32 store 32 bytes wide.  export at [12, 1000, 10000] bf16:
+// The three layout kernels below are bound by HBM.  A CTA covers 256 V columns of one layer (blockIdx.x, blockIdx.z)
+// and walks batch rows (blockIdx.y strided), so an element costs no division and the per-column parameters stay in
+// registers; V = 8 makes every load 16 and every fp32 store 32 bytes wide, V = 1 takes the rows that do not start on
+// such boundaries.  export at [12, 1000, 10000] bf16:
 // 472 -> 128 us (5.6 TB/s; 162 us with two 16-byte stores), one element per thread and step with two 64-bit divisions
 // before; act_export at [12, 333, 24576] 195 us (6.0 TB/s) for what an activation sweep and two exports took 900 us.
 
@@ -154,6 +155,19 @@ int launch_export(const void* src, const float* bias, float* out, int B, int L, 
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
+template <class T>
+int launch_act_export(const void* z, const float* bias, const float* theta, float* pre, void* feat, float* features,
+                      int B, int L, long long F, cudaStream_t s) {
+  if (F % 8 == 0 && aligned32(z) && aligned32(pre) && aligned32(feat) && aligned32(features))
+    act_export_kernel<T, 8>
+        <<<row_grid(B, L, F, 8), 256, 0, s>>>((const T*)z, bias, theta, pre, (T*)feat, features, B, L, F);
+  else
+    act_export_kernel<T, 1>
+        <<<row_grid(B, L, F, 1), 256, 0, s>>>((const T*)z, bias, theta, pre, (T*)feat, features, B, L, F);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
 // out[b, l, d] = recon[b, l, d] * sd[l, d] + mu[l, d]
 __global__ void destandardize_kernel(const float* __restrict__ recon, const float* __restrict__ mu,
                                      const float* __restrict__ sd, float* __restrict__ out, long long total, int LD) {
@@ -215,18 +229,8 @@ int clt_act_export(const void* z, const float* bias, const float* theta, float* 
                    int L, int64_t F, int bf16, clt_stream_t stream) {
   CLT_CHECK_ARG(z && bias && pre && feat && features && B > 0 && L > 0 && L <= 65535 && F > 0,
                 "act_export: bad arguments");
-  CLT_CHECK_ARG(F % 8 == 0, "act_export: d_features=%lld must be a multiple of 8", (long long)F);
-  CLT_CHECK_ARG(aligned32(z) && aligned32(pre) && aligned32(feat) && aligned32(features),
-                "act_export: buffers must be 32-byte aligned");
-  const dim3 grid = row_grid(B, L, F, 8);
-  cudaStream_t s = (cudaStream_t)stream;
-  if (bf16)
-    act_export_kernel<__nv_bfloat16, 8><<<grid, 256, 0, s>>>((const __nv_bfloat16*)z, bias, theta, pre,
-                                                             (__nv_bfloat16*)feat, features, B, L, F);
-  else
-    act_export_kernel<float, 8><<<grid, 256, 0, s>>>((const float*)z, bias, theta, pre, (float*)feat, features, B, L, F);
-  CLT_CHECK_CUDA(cudaGetLastError());
-  return 0;
+  return bf16 ? launch_act_export<__nv_bfloat16>(z, bias, theta, pre, feat, features, B, L, F, (cudaStream_t)stream)
+              : launch_act_export<float>(z, bias, theta, pre, feat, features, B, L, F, (cudaStream_t)stream);
 }
 
 int clt_import_blf(const float* src, void* dst, int B, int L, int64_t F, int bf16, clt_stream_t stream) {

@@ -16,6 +16,8 @@ CASES = [
     ("plt_jumprelu", 2, 96, 256, 77, False, "jumprelu", 0),
     ("clt_topk", 3, 64, 128, 50, True, "topk", 8),
     ("clt_batchtopk", 2, 64, 128, 64, True, "batchtopk", 4),
+    ("clt_jumprelu_odd", 2, 64, 201, 77, True, "jumprelu", 0),      # fp32 modules train at any feature count
+    ("plt_relu_odd", 3, 64, 77, 33, False, "relu", 0),
 ]
 
 
@@ -23,6 +25,8 @@ CASES = [
 @pytest.mark.parametrize("name,L,D,F,B,cross,kind,k", CASES)
 def test_kernel_forward_matches_model_forward(name, L, D, F, B, cross, kind, k, prec):
     bf16 = prec == "bf16"
+    if bf16 and F % 8:
+        pytest.skip("bf16 rows are multiples of 16 bytes")
     if bf16 and kind != "jumprelu":
         pytest.skip("selection sets of a bf16 run depend on the accumulation order; covered in fp32")
     dev = torch.device("cuda:0")
@@ -121,8 +125,7 @@ def test_layout_kernels(L, B, F, bf16):
         rows = torch.empty(B, n * F, dtype=T, device=dev)
         lib().call("clt_import_rows", x, x.stride(0), rows, B, n * F, bf16, stream_ptr())
         assert torch.equal(rows, x.to(T))
-    if F % 8 == 0:
-        want = torch.where((pre > theta) & (pre > 0), pre, torch.zeros_like(pre)).to(T)
-        p2, f2, feat = torch.empty_like(out), torch.empty_like(out), torch.empty_like(z)
-        lib().call("clt_act_export", z, bias, theta, p2, feat, f2, B, L, F, bf16, stream_ptr())
-        assert torch.equal(p2, pre) and torch.equal(f2, want.float()) and torch.equal(feat, want.transpose(0, 1))
+    want = torch.where((pre > theta) & (pre > 0), pre, torch.zeros_like(pre)).to(T)
+    p2, f2, feat = torch.empty_like(out), torch.empty_like(out), torch.empty_like(z)
+    lib().call("clt_act_export", z, bias, theta, p2, feat, f2, B, L, F, bf16, stream_ptr())
+    assert torch.equal(p2, pre) and torch.equal(f2, want.float()) and torch.equal(feat, want.transpose(0, 1))
