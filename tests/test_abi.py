@@ -178,3 +178,29 @@ def test_call_path_of_another_source_is_passed_over(tmp_path, monkeypatch):
     assert _lib._Lib()._native
     monkeypatch.setattr(build, "_C_PRELUDE", build._C_PRELUDE + "/* converts otherwise */")
     assert _lib._Lib()._native == {}
+
+
+def test_decoder_scratch_covers_the_librarys_parts():
+    """Wherever csrc/gemm.cuh (``split_blocks``, restated here) cuts the decoder's contraction axis, the step's scratch
+    holds a slab for every part, on chips of other SM counts too: too little would silently leave the chains whole."""
+    from crosslayer_transcoder_b200.engine import StepEngine
+
+    split = 0
+    for sms in (132, 148, 160):
+        for bf16 in (False, True):
+            kb, bn, slots = (64, 256, sms) if bf16 else (16, 128, 2 * sms)
+            for L in (1, 2, 3, 12, 26):
+                for crosslayer in (False, True):
+                    for B in (1, 64, 128, 129, 257, 513, 1000, 1500, 4000):
+                        for D in (64, 264, 512, 768, 2304):
+                            tiles = -(-B // 128) * -(-D // bn)
+                            slabs = StepEngine._decoder_scratch_slabs(sms, B, L, D, bf16)
+                            for F in (200, 512, 1024, 2001, 10000, 32768):
+                                chains = [(t + 1 if crosslayer else 1) * -(-F // kb) for t in range(L)]
+                                total, longest = sum(chains), max(chains)
+                                if longest < 32 or longest * slots * 2 <= total * tiles * 3:
+                                    continue
+                                part = max(8, -(-total * tiles // (2 * slots)))
+                                split += 1
+                                assert sum(-(-n // part) for n in chains) <= slabs, (sms, bf16, L, crosslayer, B, D, F)
+    assert split > 1000
