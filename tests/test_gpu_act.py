@@ -49,3 +49,22 @@ def test_streaming_activation(L, B, F, scale, bf16):
     assert close(dth, t.sum(1), t.abs().sum(1))
     w = lam * d1 * c * f
     assert close(dn, w.sum(1), w.abs().sum(1))
+
+
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_penalty_values_across_the_seam(bf16):
+    """Single values of the streaming kernel's tanh on both sides of 0.7, where it leaves its polynomial for tanhf: one live
+    feature, whose penalty is the whole sum.  The polynomial was fitted to 0.74 ulp, tanhf is specified to 2."""
+    dev, T = "cuda:0", torch.bfloat16 if bf16 else torch.float32
+    v = torch.cat([torch.logspace(-30, -2, 15), torch.linspace(0.02, 0.69, 68), torch.linspace(0.695, 0.705, 41),
+                   torch.tensor([0.7, 0.71, 0.75, 1.0, 3.0, 9.0, 30.0, float("inf")])]).to(T).float().unique().to(dev)
+    z = torch.full((v.numel(), 8), -1.0, dtype=T, device=dev)
+    z[:, 3] = v.to(T)
+    zero, one, acc = (torch.zeros(8, device=dev), torch.ones(8, device=dev), torch.zeros(v.numel(), 2, device=dev))
+    feat = torch.empty(8, dtype=T, device=dev)
+    for row, a in zip(z, acc):
+        lib().call("clt_act_fwd", row, zero, None, one, feat, None, a, 1.0, 1, 0, 1, 1, 8, bf16, stream_ptr())
+    want = torch.tanh(v.double())
+    ulp = torch.ldexp(torch.ones_like(want), torch.frexp(want).exponent - 24)
+    assert bool(((acc[:, 1].double() - want).abs() <= 2.0 * ulp).all())
+    assert bool((acc[:, 0] == 0).all())

@@ -85,16 +85,30 @@ def test_split_decoder(L, B, D, F, cross, bf16):
         _close(split[:, t], want, mag, fd.shape[0] * F)
 
 
-# 256-row tiles of CTA pairs (the batch large enough, rounding it up to 256 rows cheap) and 128-row tiles, with ragged
-# ends in every axis; a contraction of a few elements, one of one stage, one of more stages than the ring holds
-@pytest.mark.parametrize("L,B,D,F", [(2, 2049, 264, 2056), (1, 4000, 776, 3000), (3, 1281, 8, 4104), (3, 1100, 64, 2312),
-                                     (2, 300, 520, 1032), (12, 256, 256, 2048)])
-def test_bf16_products(L, B, D, F):
+def _takes_pairs(M, N, Kseg, nz):
+    """csrc/gemm_tc.cuh, use_pair"""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n, single, pairs = -(-N // 256) * nz, -(-M // 128), -(-M // 256)
+    return Kseg > 9 * 64 and pairs * n >= sms // 2 and pairs * 16 <= single * 9
+
+
+# 128-row tiles and 256-row tiles of CTA pairs (`pairs`: which of encoder, feature gradient, decoder, decoder weight and
+# encoder weight gradient take them), with ragged ends in every axis; contractions of a few elements, of one stage, of
+# more stages than the ring holds; pairs whose second CTA has part of its 128 rows (1999) or none (2049, one row in the
+# first), over several segments that each end inside a stage
+@pytest.mark.parametrize("L,B,D,F,pairs", [(2, 2049, 264, 2056, ""), (1, 4000, 776, 3000, "ef"), (3, 1281, 8, 4104, "w"),
+                                           (3, 1100, 64, 2312, ""), (2, 300, 520, 1032, ""), (12, 256, 256, 2048, ""),
+                                           (3, 1999, 1016, 2008, "efdwx"), (3, 2049, 1016, 2008, "efdwx"),
+                                           (4, 2049, 776, 1000, "efdw")])
+def test_bf16_products(L, B, D, F, pairs):
     dev = "cuda:0"
     g = torch.Generator(device=dev).manual_seed(B)
     s, st = stream_ptr(), torch.zeros(1, dtype=torch.int32, device=dev)
     bf = torch.bfloat16
     P = L * (L + 1) // 2
+    # the sizes are there for the forms that they take: a change of the rule has to bring others
+    forms = {"e": (B, F, D, L), "f": (B, F, D, L), "d": (B, D, F, L), "w": (F, D, B, P), "x": (D, F, B, L)}
+    assert "".join(k for k, m in forms.items() if _takes_pairs(*m)) == pairs
     x, W, feat, dr = (_rand(g, *n).to(bf) for n in ((L, B, D), (L, D, F), (L, B, F), (L, B, D)))
     Wd, b = _rand(g, P, F, D).to(bf), _rand(g, L, D)
 
@@ -123,3 +137,59 @@ def test_bf16_products(L, B, D, F):
             _close(dW[l * (l + 1) // 2 + q], *mm(feat[q].t(), dr[l]), B)
         blk = torch.cat([Wd[t * (t + 1) // 2 + l] for t in range(l, L)], dim=1)
         rounded(df[l], *mm(dr[l:].transpose(0, 1).reshape(B, -1), blk.t()), (L - l) * D)
+
+
+# the (Jump)ReLU and row-coefficient epilogues on the large tiles: 128 x 128 (encoder; per-layer feature gradient; weight
+# gradient) and 128 x 64 (crosslayer feature gradient), with and without 16-byte rows
+@pytest.mark.parametrize("L,B,D,F,cross", [(2, 1100, 648, 1160, 1), (2, 1101, 645, 1163, 0)])
+def test_fp32_fused_epilogues(L, B, D, F, cross):
+    dev, s = "cuda:0", stream_ptr()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert sms <= -(-B // 128) * -(-F // 128) * L < 8 * sms     # the large tiles' range of sizes (csrc/gemm_simt.cuh)
+    g = torch.Generator(device=dev).manual_seed(F)
+    P = L * (L + 1) // 2 if cross else L
+    x, W, b = _rand(g, L, B, D), _rand(g, L, D, F) * D ** -0.5, _rand(g, L, F) * 0.1
+    theta, norm = (torch.rand(L, F, generator=g, device=dev) * 0.3 for _ in range(2))
+    c, lam, pal, bw = 0.7, 0.3, 0.05, 0.5
+    z, feat, dpre = (torch.empty(L, B, F, device=dev) for _ in range(3))
+    fired, acc = torch.zeros(L, (F + 31) // 32, dtype=torch.int32, device=dev), torch.zeros(2, device=dev)
+    lib().call("clt_encoder_fwd_act", x, W, b, theta, norm, z, feat, fired, acc, c, 1, 1, B, L, D, F, 0, None, s)
+    _close(z, x.double() @ W.double(), x.double().abs() @ W.double().abs(), D)
+    pre = z + b[:, None]                               # the kernel's own fp32 sum decides every comparison
+    f32 = torch.where((pre > theta[:, None]) & (pre > 0), pre, torch.zeros_like(pre))
+    assert torch.equal(feat, f32)
+    i = torch.arange(F, device=dev)
+    assert torch.equal(((fired[:, i // 32] >> (i % 32)) & 1).bool(), (f32 > 0).any(dim=1))
+    f, n = f32.double(), norm.double()[:, None] * c
+    tw = torch.tanh(f * n)
+    # sums of n terms with about 1e-7 relative error each, added in fp32 groups
+    assert abs(float(acc[0]) - float(torch.relu(-pre.double()).sum())) <= 4e-6 * float(acc[0])
+    assert abs(float(acc[1]) - float(tw.sum())) <= 4e-6 * float(tw.sum())
+
+    dr, Wd = _rand(g, L, B, D) * 0.1, _rand(g, P, F, D) * D ** -0.5
+    dth, db, dn = (torch.zeros(L, F, device=dev) for _ in range(3))
+    lib().call("clt_decoder_dense_bwd_dfeat", dr, Wd, z, b, theta, norm, dpre, dth, db, dn, bw, lam, c, pal, 1, None, B, L,
+               D, F, cross, 0, None, s)
+    pair = lambda t, q: t * (t + 1) // 2 + q if cross else t
+    targets = lambda q: range(q, L) if cross else (q,)
+    gr, mag = (torch.stack([sum(fn(dr[t].double()) @ fn(Wd[pair(t, q)].double()).t() for t in targets(q))
+                            for q in range(L)]) for fn in (lambda v: v, torch.abs))
+    err = 2.0 ** -24 * (4.0 + 2.0 * (L * D) ** 0.5) * mag       # of the product, as in _close
+    d1 = 1 - tw * tw
+    gs = gr + lam * d1 * n
+    want = torch.where(pre >= 0, gs, torch.zeros_like(gs)) - pal * (pre < 0)
+    assert bool(((dpre.double() - want).abs() <= err + 1e-6 * want.abs() + 1e-6).all())
+    close = lambda a, w, e: bool(((a.double() - w.sum(1)).abs() <= e.sum(1) + 4e-6 * w.abs().sum(1) + 1e-6).all())
+    d = pre - theta[:, None]
+    rect = (d > -0.5 * bw) & ~(d > 0.5 * bw)
+    slope = theta.double()[:, None] / bw
+    assert close(db, want, err)
+    assert close(dth, torch.where(rect, -slope * gs, torch.zeros_like(gs)), slope * err)
+    assert close(dn, lam * d1 * c * f, torch.zeros_like(f))
+
+    coef, dW = _rand(g, L, F) * 0.1, torch.empty(P, F, D, device=dev)
+    lib().call("clt_decoder_dense_bwd_dw", feat, dr, dW, coef, Wd, B, L, D, F, cross, 0, None, s)
+    for t in range(L):
+        for q in range(t + 1) if cross else (t,):
+            add = coef[q].double()[:, None] * Wd[pair(t, q)].double()
+            _close(dW[pair(t, q)], f[q].t() @ dr[t].double() + add, f[q].t() @ dr[t].double().abs() + add.abs(), B)
