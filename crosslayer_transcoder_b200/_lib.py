@@ -104,6 +104,10 @@ class _Lib:
                 raise CltError(self.last_error())
             self._device_ok.add(dev)
 
+    def query(self, name: str, *args) -> int:
+        """The value of an entry point that launches nothing and cannot fail."""
+        return (self._native.get(name) or self._fn[name])(*args)
+
     def call(self, name: str, *args):
         """Call an ``int``-returning entry point; tensors are passed as their data pointers."""
         native = self._native.get(name)

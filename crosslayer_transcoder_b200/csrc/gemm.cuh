@@ -42,7 +42,7 @@ __host__ __device__ inline void pair_split(int p, int& t, int& s) {
   s = p - tt * (tt + 1) / 2;
 }
 
-// Slabs are visited longest-first so that a static round-robin over CTAs ends evenly.
+// Slabs are visited longest-first, so that the chains that are dealt last are short.
 __host__ __device__ inline int slab_of_rank(const GemmGeom& g, int rank) {
   return g.mode == kDecFwd ? g.nz - 1 - rank : rank;
 }
@@ -77,7 +77,8 @@ __host__ __device__ inline void seg_index(const GemmGeom& g, int z, int j, int& 
 }
 
 // Split-K.  The contraction of slab z, counted in the kernel's k-blocks (kb_per_seg to a segment), is cut into
-// parts of kb_per_part blocks, numbered slab by slab; part i writes its partial sums to output slab i.
+// parts of kb_per_part blocks, numbered slab by slab; part i writes its partial sums to output slab i.  (Where it is worth
+// it is decided beside the entry point, gemm_dense.cu.)
 __host__ __device__ inline int part_count(const GemmGeom& g, int z, int kb_per_seg) {
   return (seg_count(g, z) * kb_per_seg + g.kb_per_part - 1) / g.kb_per_part;
 }
@@ -98,24 +99,6 @@ __host__ __device__ inline void work_item(const GemmGeom& g, int rank, int kb_pe
   lo = rank * g.kb_per_part;
   hi = seg_count(g, z) * kb_per_seg;
   if (hi > lo + g.kb_per_part) hi = lo + g.kb_per_part;
-}
-
-// Blocks per part for a launch whose longest chain of k-blocks would outlast its fair share of the chip, 0 to
-// leave it whole.  `tiles` output tiles per slab run `slots` at a time, so a fair share is total * tiles / slots
-// blocks.  A chain may be 3/2 of that: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) the whole chains
-// took 170 us and parts 200 us; at 1.9 (fp32, 24 tiles, 1 to 12 segments of 64 blocks) 1784 and 1460 us; 9 tiles with
-// chains of 157 to 1884 blocks (12 calls) 4604 and 568 us.  Parts of half a share keep the last wave short; below
-// 8 blocks a part's output costs more than its products.
-inline int split_blocks(const GemmGeom& g, long long tiles, int kb_per_seg, int slots) {
-  long long total = 0, longest = 0;
-  for (int z = 0; z < g.nz; ++z) {
-    const long long n = (long long)seg_count(g, z) * kb_per_seg;
-    total += n;
-    longest = n > longest ? n : longest;
-  }
-  if (longest < 32 || longest * slots * 2 <= total * tiles * 3) return 0;
-  const long long part = (total * tiles + 2 * slots - 1) / (2 * slots);
-  return (int)(part < 8 ? 8 : part);
 }
 
 }  // namespace clt

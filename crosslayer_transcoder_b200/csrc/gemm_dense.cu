@@ -60,6 +60,58 @@ int run_gemm(const GemmGeom& g, const Operand& a, const Operand& b, const typena
 
 bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F > 0; }
 
+// Cuts the decoder's contraction axis into parts (gemm.cuh) where that is faster; sets g.kb_per_part and returns the
+// number of parts, or 0 for whole chains.
+//
+// Output tiles run `slots` at a time (one to an SM in bf16, two in fp32), so a fair share of the work is
+// total * tiles / slots k-blocks, and the launch lasts as long as its longest chain.  Parts come into question when that
+// chain is over 3/2 of the share: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) whole chains took 170 us and
+// parts 200 us.  Parts of half a share keep the last wave short; below 8 blocks a part's output costs more than its
+// products.  Then both forms are estimated (us):
+//   * a bf16 block takes its CTA 0.39 (staging its operands from L2), whatever the tile is filled with;
+//   * fp32: 2.2 in a 128 x 128 tile, two to an SM, 0.62 of the SM's time in a 64 x 64 tile but 0.9 of its own; small
+//     tiles are what whole chains get when the large ones are fewer than the SMs, and what parts often are not;
+//   * the weights cross HBM once at 5.5 TB/s;
+//   * parts add a launch and their sums' way to memory and back: 6 us and 8 bytes each at 5 TB/s.
+// 430 random sizes of 5 to 1500 tokens, 64 to 2304 wide, whole -> parts: 9 tiles with chains of 157 to 1884 blocks (12
+// calls) 4604 -> 568 us, fp32 24 tiles of 1 to 12 segments 1784 -> 1460; none that is taken is slower by more than
+// 2 %, and none that is left whole would have gained more than a fifth.  By the 3/2 alone 14 of them lost 3 to 50 % (short
+// chains over many tokens: 8 layers x 528 tokens x 512 wide, 35 blocks 29.6 -> 44.0 us; few tokens in fp32: 8 x 43 x 2296,
+// 591 blocks 716 -> 976 us).
+int plan_parts(GemmGeom& g, bool bf16, int sms) {
+  const auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const int kb = bf16 ? tc::kBK : kSimtBK, kb_per_seg = (int)up(g.Kseg, kb);
+  const long long tiles = up(g.M, 128) * up(g.N, bf16 ? tc::kBN : 128), slots = bf16 ? sms : 2 * sms;
+  long long total = 0, longest = 0;
+  for (int z = 0; z < g.nz; ++z) {
+    const long long n = (long long)seg_count(g, z) * kb_per_seg;
+    total += n;
+    longest = n > longest ? n : longest;
+  }
+  if (longest < 32 || longest * slots * 2 <= total * tiles * 3) return 0;
+  const long long half = up(total * tiles, 2 * slots), part = half < 8 ? 8 : half;
+  g.kb_per_part = (int)part;
+  long long parts = 0;
+  for (int z = 0; z < g.nz; ++z) parts += part_count(g, z, kb_per_seg);
+  double whole, split;
+  if (bf16) {
+    whole = 0.39 * longest;
+    split = 0.39 * part * up(parts * tiles, slots);
+  } else {
+    const long long small = up(g.M, 64) * up(g.N, 64);
+    whole = tiles * g.nz < sms ? fmax(0.9 * longest, 0.62 * total * small / sms) : 2.2 * longest;
+    split = parts * tiles < sms ? part * fmax(0.9, 0.62 * up(parts * small, sms)) : 2.2 * part * up(parts * tiles, slots);
+  }
+  const double weights = (double)total * kb * g.N * (bf16 ? 2 : 4) / 5.5e6;
+  split = fmax(split, weights) + 6.0 + 8.0 * parts * g.M * g.N / 5e6;
+  if (parts > 65535 || 1.05 * split >= fmax(whole, weights)) return g.kb_per_part = 0;
+  return (int)parts;
+}
+
+GemmGeom decoder_geom(int B, int L, int D, int F, int crosslayer) {
+  return GemmGeom{crosslayer ? kDecFwd : kBatched, B, D, F, L, L};
+}
+
 // recon[b, t, d] = b_dec[t, d] + the partial sums of target t's parts, in their order.  V consecutive d per thread.
 template <int V>
 __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ ws, const float* __restrict__ b_dec,
@@ -135,38 +187,38 @@ int clt_decoder_dense_fwd_ws(const void* feat, const void* W_dec, const float* b
   CLT_CHECK_ARG(dims_ok(B, L, D, F), "decoder_dense_fwd: bad dims B=%d L=%d D=%d F=%d", B, L, D, F);
   CLT_CHECK_ARG(feat && W_dec && recon, "decoder_dense_fwd: null pointer");
   const int P = crosslayer ? L * (L + 1) / 2 : L;
-  GemmGeom g{crosslayer ? kDecFwd : kBatched, B, D, F, L, L};
+  GemmGeom g = decoder_geom(B, L, D, F, crosslayer);
   Operand a{feat, 1, B, F, L}, b{W_dec, 0, D, F, P};
-  epi::DecOut::Params p{recon, b_dec, (long long)L * D, (long long)D};
   if (ws != nullptr) {
     CLT_CHECK_ARG((uintptr_t)ws % 16 == 0, "decoder_dense_fwd: the workspace must be 16-byte aligned");
-    const int kb = bf16 ? tc::kBK : kSimtBK, kb_per_seg = (F + kb - 1) / kb;
-    // output tiles of a slab, and how many of them the chip works on at once (the fp32 kernel runs two to an SM)
-    const int bn = bf16 ? tc::kBN : 128;
-    const long long tiles = (long long)((B + 127) / 128) * ((D + bn - 1) / bn);
-    g.kb_per_part = split_blocks(g, tiles, kb_per_seg, device_sm_count() * (bf16 ? 1 : 2));
-    if (g.kb_per_part > 0) {
-      long long parts = 0;
-      for (int t = 0; t < L; ++t) parts += part_count(g, t, kb_per_seg);
-      if (parts * B * D <= ws_floats && parts <= 65535) {
-        g.nz = (int)parts;
-        epi::DecOut::Params pp{ws, nullptr, (long long)D, (long long)B * D};
-        if (int rc = run_gemm<epi::DecOut, epi::DecOut, false, true>(g, a, b, pp, pp, bf16, status, (cudaStream_t)stream)) return rc;
-        const long long slab = (long long)B * D;
-        if (D % 4 == 0 && ((uintptr_t)recon | (uintptr_t)b_dec) % 16 == 0) {
-          sum_parts_kernel<4><<<dim3((unsigned)((slab / 4 + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
-              ws, b_dec, recon, g, kb_per_seg);
-        } else {
-          sum_parts_kernel<1><<<dim3((unsigned)((slab + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
-              ws, b_dec, recon, g, kb_per_seg);
-        }
-        CLT_CHECK_CUDA(cudaGetLastError());
-        return 0;
+    const long long slab = (long long)B * D;
+    const int parts = plan_parts(g, bf16 != 0, device_sm_count());
+    if (parts > 0 && parts * slab <= ws_floats) {
+      g.nz = parts;
+      epi::DecOut::Params pp{ws, nullptr, (long long)D, slab};
+      if (int rc = run_gemm<epi::DecOut, epi::DecOut, false, true>(g, a, b, pp, pp, bf16, status, (cudaStream_t)stream))
+        return rc;
+      const int kb = bf16 ? tc::kBK : kSimtBK, kb_per_seg = (F + kb - 1) / kb;
+      if (D % 4 == 0 && ((uintptr_t)recon | (uintptr_t)b_dec) % 16 == 0) {
+        sum_parts_kernel<4><<<dim3((unsigned)((slab / 4 + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
+            ws, b_dec, recon, g, kb_per_seg);
+      } else {
+        sum_parts_kernel<1><<<dim3((unsigned)((slab + 255) / 256), L), 256, 0, (cudaStream_t)stream>>>(
+            ws, b_dec, recon, g, kb_per_seg);
       }
-      g.kb_per_part = 0;  // the workspace is too small: whole chains
+      CLT_CHECK_CUDA(cudaGetLastError());
+      return 0;
     }
+    g.kb_per_part = 0;  // the workspace is too small: whole chains
   }
+  epi::DecOut::Params p{recon, b_dec, (long long)L * D, (long long)D};
   return run_gemm<epi::DecOut, epi::DecOut, false, true>(g, a, b, p, p, bf16, status, (cudaStream_t)stream);
+}
+
+int clt_decoder_dense_parts(int B, int L, int D, int F, int crosslayer, int bf16, int num_sms) {
+  if (!dims_ok(B, L, D, F)) return 0;
+  GemmGeom g = decoder_geom(B, L, D, F, crosslayer);
+  return plan_parts(g, bf16 != 0, num_sms > 0 ? num_sms : device_sm_count());
 }
 
 int clt_decoder_dense_fwd_push(const void* feat, const void* W_dec, const float* b_dec, const uint64_t* rank_bases,

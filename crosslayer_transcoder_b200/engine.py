@@ -13,7 +13,6 @@ for allocation, streams and autograd plumbing only; there is no eager fallback.
 """
 from __future__ import annotations
 
-import functools
 from typing import Dict, List, Optional
 
 import torch
@@ -22,11 +21,6 @@ from . import _lib
 from ._lib import DTYPE_CODE, CltError, lib, stream_ptr
 
 _ALIGN = 64  # elements; keeps every segment 256-byte aligned in fp32 and 128-byte aligned in bf16
-
-
-@functools.lru_cache(maxsize=None)
-def _sm_count(device: torch.device) -> int:
-    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def _round_up(n: int, a: int = _ALIGN) -> int:
@@ -416,19 +410,10 @@ class StepEngine:
         lists and for rows too wide for one warp's registers."""
         return int(k <= 8 * world or (k <= 64 and D <= 1024))
 
-    @staticmethod
-    def _decoder_scratch_slabs(sms: int, B: int, L: int, D: int, bf16: bool) -> int:
-        """[B, D] slabs of scratch with which the library may split the contraction axis of the dense decoder
-        (csrc/gemm.cuh, ``split_blocks``: at most two parts per running tile, and one rounded up per target), 0 where
-        the output tiles fill the chip.  The bf16 kernel runs one tile to an SM, the fp32 kernel two."""
-        tiles = -(-B // 128) * -(-D // (256 if bf16 else 128))
-        slots = sms if bf16 else 2 * sms
-        return 2 * slots // tiles + L + 1 if 4 * slots > 3 * (L + 1) * tiles else 0
-
     def _decoder_dense_fwd(self, feat, W, bias, recon, B, L, D, F, crosslayer, bf16, split=True):
-        """The dense decoder contraction, with scratch for partial sums where the library may want to split the
+        """The dense decoder contraction, with scratch for partial sums where the library wants to split the
         contraction axis.  The scratch is this call's own: forwards may run on several streams."""
-        n = self._decoder_scratch_slabs(_sm_count(recon.device), B, L, D, bf16) * B * D if split else 0
+        n = lib().query("clt_decoder_dense_parts", B, L, D, F, crosslayer, int(bf16), 0) * B * D if split else 0
         ws = torch.empty(n, dtype=torch.float32, device=recon.device) if n else None
         self._call("clt_decoder_dense_fwd_ws", feat, W, bias, recon, ws, n, B, L, D, F, crosslayer, int(bf16),
                    self.status, stream_ptr())

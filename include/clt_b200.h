@@ -69,10 +69,13 @@ int clt_decoder_dense_fwd(const void* feat, const void* W_dec, const float* b_de
 /* clt_decoder_dense_fwd with scratch for partial sums.  When the batch gives fewer output tiles than the chip has
  * room for, the contraction axis is cut into parts that run side by side, each writing its [B, D] partial sums to
  * ws; a second kernel adds them in a fixed order.  ws holds ws_floats floats (16-byte aligned, contents undefined
- * before and after); with ws NULL or too small every output is one chain. */
+ * before and after); with ws NULL or too small every output is one chain.
+ * clt_decoder_dense_parts returns for how many slabs of B * D floats that call has a use (0: it keeps whole chains
+ * anyway), on a chip of num_sms SMs (0: the current device).  It launches nothing. */
 int clt_decoder_dense_fwd_ws(const void* feat, const void* W_dec, const float* b_dec, float* recon, float* ws,
                              int64_t ws_floats, int B, int L, int D, int F, int crosslayer, int bf16, int* status,
                              clt_stream_t stream);
+int clt_decoder_dense_parts(int B, int L, int D, int F, int crosslayer, int bf16, int num_sms);
 
 /* clt_decoder_dense_fwd fused with the exchange of the partial reconstructions over the feature-shard
  * ranks of one node (same buffer convention as clt_sparse_decoder_fwd_push: per-source slots
