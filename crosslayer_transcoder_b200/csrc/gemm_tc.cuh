@@ -17,7 +17,7 @@
 // of B, and one tcgen05.mma.cta_group::2, issued by the even CTA, multiplies both.  That is a third less operand
 // traffic from L2 and through shared memory per product, which is what bounded the single form (40-56 % of L2 peak at
 // 78 % tensor activity): 12-layer weight gradients 1.27 -> 1.12 ms (1.35 PFLOP/s), decoder forward 0.64 -> 0.60 ms
-// (1.38), encoder 0.43 -> 0.41 ms (1.35) at 4000 tokens, and within 1 % where the power cap sets the rate.
+// (1.38), encoder 0.43 -> 0.41 ms (1.35) at 4000 tokens; whole steps, where the power cap sets the rate, 1 to 3 %.
 // Stages are handed from the producers to the MMA lane through full/empty mbarriers; the even CTA's full barrier
 // counts the bytes of both.  Two 256-column accumulators in tensor memory let the epilogue of one tile overlap the
 // main loop of the next.
@@ -46,7 +46,7 @@
 namespace clt {
 namespace tc {
 
-constexpr int kBM = 128, kBN = 256, kBK = 64;  // output rows of a CTA, columns of its tile, contraction steps of a stage
+constexpr int kBM = 128, kBN = 256, kBK = 64;  // output rows of a CTA, columns of its tile, contraction of a stage
 template <bool kPair>
 struct Tile {
   static constexpr int kCtas = kPair ? 2 : 1;
@@ -351,8 +351,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 break;
               }
               // the leader's barrier counts the bytes of both CTAs
-              const uint32_t full = kPair ? cluster_addr(smem_u32(&bars->full[stage]), 0) : smem_u32(&bars->full[stage]);
-              if (rank == 0) mbar_expect_tx(smem_u32(&bars->full[stage]), TL::kCtas * kStageBytes);
+              const uint32_t own = smem_u32(&bars->full[stage]), full = kPair ? cluster_addr(own, 0) : own;
+              if (rank == 0) mbar_expect_tx(own, TL::kCtas * kStageBytes);
               const uint32_t sa = smem_u32(smem + stage * kStageBytes);
               const uint32_t sb = sa + kABytes;
               const int k0 = kb * kBK;
@@ -364,7 +364,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
               }
               if (B_MN) {
   #pragma unroll
-                for (int i = 0; i < TL::kBRows / 64; ++i) tma_load_3d<kPair>(sb + i * 8192, &mapB, full, n0 + 64 * i, k0, zb);
+                for (int i = 0; i < TL::kBRows / 64; ++i)
+                  tma_load_3d<kPair>(sb + i * 8192, &mapB, full, n0 + 64 * i, k0, zb);
               } else {
                 tma_load_3d<kPair>(sb, &mapB, full, k0, n0, zb);
               }
@@ -559,13 +560,21 @@ struct TcOperand {
 };
 
 // Pairs of CTAs, unless rounding M up to 256 rows adds more than an eighth to the work, pairs would leave part of the
-// chip without a tile, or the chain is so short that a tile is bound by its output (then the two CTAs only wait for one
+// chip without a tile, or a tile may be so short that it is bound by its output (then the two CTAs only wait for one
 // another: weight gradients over 333 and 512 tokens 0.51 -> 0.57 and 0.100 -> 0.107 ms as pairs, over 1000 tokens
-// 0.196 -> 0.187, over 4000 tokens 1.27 -> 1.12 ms).
+// 0.196 -> 0.187, over 4000 tokens 1.27 -> 1.12 ms).  Short is judged by one segment, which for those is the whole
+// chain.  Chains of several segments are longer than that: the crosslayer feature gradient of 12 layers, 4000 tokens
+// and 10000 features, which stays single at these widths, would take 2.32 instead of 2.35 ms as pairs at 512, 1.18
+// instead of 1.32 at 256.  Parts of a chain (kb_per_part) are shorter: at 8 blocks both forms take 40 to 64 us, within
+// 7 % of each other either way.
+// Nor are pairs taken where they need more rounds of the chip than singles and the difference is over a tenth, which is
+// what a pair is faster by: 5 rounds for 4 took 54 instead of 45 us (encoder, 2 x 1083 x 1072 x 7840), 11 for 10 take
+// 0.84 to 0.86 of the time.
 inline bool use_pair(const GemmGeom& g, int num_sms) {
   const long long n_tiles = (g.N + kBN - 1) / kBN, single = (long long)((g.M + kBM - 1) / kBM) * n_tiles * g.nz;
   const long long pairs = (long long)((g.M + 2 * kBM - 1) / (2 * kBM)) * n_tiles * g.nz;
-  return g.Kseg > 9 * kBK && pairs >= num_sms / 2 && pairs * 16 <= single * 9;
+  const long long rounds = (single + num_sms - 1) / num_sms, pair_rounds = (pairs + num_sms / 2 - 1) / (num_sms / 2);
+  return g.Kseg > 9 * kBK && pairs >= num_sms / 2 && pairs * 16 <= single * 9 && pair_rounds * 9 <= rounds * 10;
 }
 
 int encode_operand_map(CUtensorMap* map, const TcOperand& o, int tile_rows_if_k_major);

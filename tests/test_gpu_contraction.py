@@ -88,8 +88,10 @@ def test_split_decoder(L, B, D, F, cross, bf16):
 def _takes_pairs(M, N, Kseg, nz):
     """csrc/gemm_tc.cuh, use_pair"""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    n, single, pairs = -(-N // 256) * nz, -(-M // 128), -(-M // 256)
-    return Kseg > 9 * 64 and pairs * n >= sms // 2 and pairs * 16 <= single * 9
+    n = -(-N // 256) * nz
+    single, pairs = -(-M // 128) * n, -(-M // 256) * n
+    rounds, pair_rounds = -(-single // sms), -(-pairs // (sms // 2))
+    return Kseg > 9 * 64 and pairs >= sms // 2 and pairs * 16 <= single * 9 and pair_rounds * 9 <= rounds * 10
 
 
 # 128-row tiles and 256-row tiles of CTA pairs (`pairs`: which of encoder, feature gradient, decoder, decoder weight and
@@ -99,7 +101,7 @@ def _takes_pairs(M, N, Kseg, nz):
 @pytest.mark.parametrize("L,B,D,F,pairs", [(2, 2049, 264, 2056, ""), (1, 4000, 776, 3000, "ef"), (3, 1281, 8, 4104, "w"),
                                            (3, 1100, 64, 2312, ""), (2, 300, 520, 1032, ""), (12, 256, 256, 2048, ""),
                                            (3, 1999, 1016, 2008, "efdwx"), (3, 2049, 1016, 2008, "efdwx"),
-                                           (4, 2049, 776, 1000, "efdw")])
+                                           (4, 2049, 776, 1000, "efdw"), (2, 1083, 1072, 7840, "w")])
 def test_bf16_products(L, B, D, F, pairs):
     dev = "cuda:0"
     g = torch.Generator(device=dev).manual_seed(B)
