@@ -614,41 +614,46 @@ int loss_bwd(const float* recon, const float* aux, const void* batch, int in_dty
 // A thread owns 8 consecutive features: their bias / threshold / norm live in registers, the
 // per-feature sums accumulate in registers over the CTA's rows and leave with one atomic each.
 //
-// Bound by HBM once enough rows are in flight: kActRows rows of a thread's columns are loaded before the first is
-// used.  12 x 4000 x 24576 bf16: forward 1040 -> 860 us (5.5 TB/s), backward 1900 -> 1275 us (5.6 TB/s) against one row
-// at a time.
+// Bound by HBM once enough rows are in flight: two to four rows of a thread's columns are loaded before the first is
+// used.  12 x 4000 x 10000 bf16 without penalty: forward 483 -> 358 us (5.4 TB/s), backward 862 -> 563 us (5.1 TB/s)
+// against one row at a time.  fp32 forward, 12 x 512 x 4096 with penalty, one row -> two -> four: 70 -> 54 -> 46 us.
 //
 // forward : feat = pre [pre > theta, pre > 0], pre = z + b;  loss_acc[0] += sum relu(-pre),
 //           loss_acc[1] += sum tanh(feat n c) (or the product);  fired bits
 // backward: dpre, dtheta, db_enc, d dec_norm from g = dL/dfeat exactly as csrc/epilogues.cuh states
 // ---------------------------------------------------------------------------------
+constexpr int kFwdRows = 4;
 template <class T>
-constexpr int kActRows = sizeof(T) == 2 ? 4 : 2;  // the same bytes in flight
+constexpr int kBwdRows = sizeof(T) == 2 ? 4 : 2;  // two streams: four fp32 rows of both do not fit the registers
 
 // tanh of 8 values.  tanhf branches for every value, which keeps the eight from overlapping and made the sweeps with a
-// sparsity penalty issue-bound.  Here one branch covers all eight: below 0.7 (where penalties live: feature x decoder norm x c)
-// tanh(x) = x + x^3 P(x^2), P of degree 5 fitted by iteratively reweighted least squares to the smallest largest
-// relative error (7e-10; in fp32 0.74 ulp against float64, tanhf is specified to 2); anything larger takes tanhf.
-// 12 x 4000 x 10000 bf16 with penalty: forward 745 -> 660 us, backward 1370 -> 1210 us.
+// sparsity penalty issue-bound.  Here one branch covers all eight: below 0.7 (where penalties live: feature x decoder
+// norm x c) tanh(x) = x + x^3 P(x^2), P of degree 5 fitted by iteratively reweighted least squares to the smallest
+// largest relative error (3.7e-9 with the coefficients as rounded to fp32; evaluated in fp32 0.74 ulp against float64,
+// tanhf is specified to 2); anything larger takes tanhf, and only that: with the polynomial in front of the branch
+// saturated penalties paid for both, and the backward sweep spilled registers.
+// 12 x 4000 x 10000 bf16, a row and tanhf at a time -> four rows, polynomial in front -> here: forward 629 -> 498 -> 449
+// us and backward 1316 -> 879 -> 872 for penalties below 0.7, 629 -> 684 -> 586 and 1311 -> 1118 -> 999 where all are
+// saturated, 629 -> 690 -> 674 and 1313 -> 1120 -> 1094 where every warp has both.
 __device__ __forceinline__ void tanh8(float (&v)[8]) {
-  float top = 0.f, t[8];
+  float top = 0.f;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float s = v[q] * v[q];
-    top = fmaxf(top, s);
-    float p = fmaf(s, 0.001895663677714765f, -0.007883304730057716f);
-    p = fmaf(s, p, 0.02157105877995491f);
-    p = fmaf(s, p, -0.05392095446586609f);
-    p = fmaf(s, p, 0.133329838514328f);
-    p = fmaf(s, p, -0.33333325386047363f);
-    t[q] = fmaf(p, v[q] * s, v[q]);
+  for (int q = 0; q < 8; ++q) top = fmaxf(top, fabsf(v[q]));
+  if (top > 0.7f) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = tanhf(v[q]);
+  } else {  // (a NaN among them comes here, and through)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float s = v[q] * v[q];
+      float p = fmaf(s, 0.001895663677714765f, -0.007883304730057716f);
+      p = fmaf(s, p, 0.02157105877995491f);
+      p = fmaf(s, p, -0.05392095446586609f);
+      p = fmaf(s, p, 0.133329838514328f);
+      p = fmaf(s, p, -0.33333325386047363f);
+      v[q] = fmaf(p, v[q] * s, v[q]);
+    }
   }
-  if (top > 0.49f) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) t[q] = tanhf(v[q]);
-  }
-#pragma unroll
-  for (int q = 0; q < 8; ++q) v[q] = t[q];
 }
 
 template <class T>
@@ -694,12 +699,12 @@ act_fwd_kernel(const T* __restrict__ z, const float* __restrict__ b_enc, const f
     };
     size_t o = ((size_t)l * B + r0) * F + f0;
     int r = r0;
-    for (; r + kActRows<T> <= r1; r += kActRows<T>) {
-      Raw8<T> zr[kActRows<T>];
+    for (; r + kFwdRows <= r1; r += kFwdRows) {
+      Raw8<T> zr[kFwdRows];
 #pragma unroll
-      for (int i = 0; i < kActRows<T>; ++i) zr[i].load(z + o + (size_t)i * F);
+      for (int i = 0; i < kFwdRows; ++i) zr[i].load(z + o + (size_t)i * F);
 #pragma unroll
-      for (int i = 0; i < kActRows<T>; ++i, o += F) row(zr[i], o);
+      for (int i = 0; i < kFwdRows; ++i, o += F) row(zr[i], o);
     }
     for (; r < r1; ++r, o += F) {
       Raw8<T> zr;
@@ -785,12 +790,12 @@ act_bwd_kernel(const T* g, const T* __restrict__ z, const float* __restrict__ b_
   // g and dpre may be one buffer: a thread writes only elements that it has read
   size_t o = ((size_t)l * B + r0) * F + f0;
   int r = r0;
-  for (; r + kActRows<T> <= r1; r += kActRows<T>) {
-    Raw8<T> gr[kActRows<T>], zr[kActRows<T>];
+  for (; r + kBwdRows<T> <= r1; r += kBwdRows<T>) {
+    Raw8<T> gr[kBwdRows<T>], zr[kBwdRows<T>];
 #pragma unroll
-    for (int i = 0; i < kActRows<T>; ++i) gr[i].load(g + o + (size_t)i * F), zr[i].load(z + o + (size_t)i * F);
+    for (int i = 0; i < kBwdRows<T>; ++i) gr[i].load(g + o + (size_t)i * F), zr[i].load(z + o + (size_t)i * F);
 #pragma unroll
-    for (int i = 0; i < kActRows<T>; ++i, o += F) row(gr[i], zr[i], o);
+    for (int i = 0; i < kBwdRows<T>; ++i, o += F) row(gr[i], zr[i], o);
   }
   for (; r < r1; ++r, o += F) {
     Raw8<T> gr, zr;
@@ -806,7 +811,7 @@ act_bwd_kernel(const T* g, const T* __restrict__ z, const float* __restrict__ b_
   }
 }
 
-// long enough columns that the sums' atomics and the parameters' loads do not count, a multiple of kActRows
+// long enough columns that the sums' atomics and the parameters' loads do not count, a multiple of kBwdRows
 static int act_rows_per_cta(int B) { return B >= 2048 ? 128 : (B >= 256 ? 64 : 16); }
 
 int act_fwd(const void* z, const float* b_enc, const float* theta, const float* dec_norm, void* feat,
