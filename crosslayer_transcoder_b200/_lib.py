@@ -116,7 +116,7 @@ class _Lib:
             try:
                 rc = native(*args)
             except TypeError:
-                pass                    # nothing was called: ctypes takes its own pointer objects, or says what is wrong
+                pass            # nothing was called: ctypes takes its own pointer objects, or says what is wrong
         if rc is None:
             rc = self._fn[name](*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args])
         if rc != 0:

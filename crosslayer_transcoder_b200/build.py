@@ -77,9 +77,9 @@ static int as_f32(PyObject* a, float* out) {
 
 
 def binding_source(protos):
-    """(digest, text): C source of the ``_clt_call`` extension module for ``_lib.parse_header``'s prototypes.  ``bind(name, address)``
-    gives a wrapper its entry point; a wrapper raises TypeError before it calls anything.  The module's
-    ``source`` is the digest, so that one which was made from another text is recognised."""
+    """(digest, text): C source of the ``_clt_call`` extension module for ``_lib.parse_header``'s prototypes.
+    ``bind(name, address)`` gives a wrapper its entry point; a wrapper raises TypeError before it calls anything.  The
+    module's ``source`` is the digest, so that one which was made from another text is recognised."""
     kinds = {ctypes.c_void_p: ("void*", "void*", "as_ptr"), ctypes.c_int: ("int", "int64_t", "as_i64"),
              ctypes.c_int64: ("int64_t", "int64_t", "as_i64"), ctypes.c_float: ("float", "float", "as_f32")}
     names = [n for n, (ret, args) in protos.items() if ret is ctypes.c_int and args]

@@ -70,8 +70,8 @@ struct ToFloat<__nv_bfloat16> {
 
 // 8 consecutive fp32 values of a lane as one 32-byte store (p a multiple of 32 bytes).  Two 16-byte stores at a lane
 // distance of 32 bytes touch every sector of the warp's kilobyte twice, half of it each time: encoder gradients
-// of the sparse steps 489 -> 383, 1000 -> 865 and 310 -> 248 us.  (The decoder pass with the optimizer, whose three streams
-// are read as well, is 3 % slower with 32-byte accesses and keeps 16.)
+// of the sparse steps 489 -> 383, 1000 -> 865 and 310 -> 248 us.  (The decoder pass with the optimizer, whose three
+// streams are read as well, is 3 % slower with 32-byte accesses and keeps 16.)
 __device__ __forceinline__ void st_f32x8(float* p, const float4& a, const float4& b) {
   asm volatile("st.global.cs.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
                "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(p)

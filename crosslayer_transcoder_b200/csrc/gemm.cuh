@@ -77,8 +77,8 @@ __host__ __device__ inline void seg_index(const GemmGeom& g, int z, int j, int& 
 }
 
 // Split-K.  The contraction of slab z, counted in the kernel's k-blocks (kb_per_seg to a segment), is cut into
-// parts of kb_per_part blocks, numbered slab by slab; part i writes its partial sums to output slab i.  (Where it is worth
-// it is decided beside the entry point, gemm_dense.cu.)
+// parts of kb_per_part blocks, numbered slab by slab; part i writes its partial sums to output slab i.  (Whether that
+// is worth it is decided beside the entry point, gemm_dense.cu.)
 __host__ __device__ inline int part_count(const GemmGeom& g, int z, int kb_per_seg) {
   return (seg_count(g, z) * kb_per_seg + g.kb_per_part - 1) / g.kb_per_part;
 }

@@ -53,7 +53,8 @@ int run_gemm(const GemmGeom& g, const Operand& a, const Operand& b, const typena
   if (bf16) {
     CLT_CHECK_ARG(status != nullptr, "the tensor-core path needs a device status word");
     CLT_CHECK_ARG(a.k_contig == (A_MN ? 0 : 1) && b.k_contig == (B_MN ? 0 : 1), "gemm: operand layout");
-    return tc::launch_gemm_tc<EpiBf16, A_MN, B_MN>(g, tc_operand(a), tc_operand(b), p16, status, device_sm_count(), stream);
+    return tc::launch_gemm_tc<EpiBf16, A_MN, B_MN>(g, tc_operand(a), tc_operand(b), p16, status, device_sm_count(),
+                                                   stream);
   }
   return launch_gemm_simt<EpiF32>(g, simt_operands(a, b), p32, device_sm_count(), stream);
 }
@@ -64,20 +65,24 @@ bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F >
 // number of parts, or 0 for whole chains.
 //
 // Output tiles run `slots` at a time (one to an SM in bf16, two in fp32), so a fair share of the work is
-// total * tiles / slots k-blocks, and the launch lasts as long as its longest chain.  Parts come into question when that
-// chain is over 3/2 of the share: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) whole chains took 170 us and
-// parts 200 us.  Parts of half a share keep the last wave short; below 8 blocks a part's output costs more than its
+// total * tiles / slots k-blocks, and the launch lasts as long as its longest chain.  Parts come into question when
+// that chain is over 3/2 of the share: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) whole chains took 170
+// us and parts 200 us.  Parts of half a share keep the last wave short; below 8 blocks a part's output costs more than its
 // products.  Then both forms are estimated (us):
 //   * a bf16 block takes its CTA 0.39 (staging its operands from L2), whatever the tile is filled with;
 //   * fp32: 2.2 in a 128 x 128 tile, two to an SM, 0.62 of the SM's time in a 64 x 64 tile but 0.9 of its own; small
-//     tiles are what whole chains get when the large ones are fewer than the SMs, and what parts often are not;
+//     tiles are what whole chains get when the large ones are fewer than the SMs, and what parts often do not get;
 //   * the weights cross HBM once at 5.5 TB/s;
 //   * parts add a launch and their sums' way to memory and back: 6 us and 8 bytes each at 5 TB/s.
 // 430 random sizes of 5 to 1500 tokens, 64 to 2304 wide, whole -> parts: 9 tiles with chains of 157 to 1884 blocks (12
 // calls) 4604 -> 568 us, fp32 24 tiles of 1 to 12 segments 1784 -> 1460; none that is taken is slower by more than
-// 2 %, and none that is left whole would have gained more than a fifth.  By the 3/2 alone 14 of them lost 3 to 50 % (short
-// chains over many tokens: 8 layers x 528 tokens x 512 wide, 35 blocks 29.6 -> 44.0 us; few tokens in fp32: 8 x 43 x 2296,
-// 591 blocks 716 -> 976 us).
+// 2 %, and none that is left whole would have gained more than a fifth.  By the 3/2 alone over a dozen lost 10 to 50 %
+// (short chains over many tokens: 8 layers x 528 tokens x 512 wide, 35 blocks 29.6 -> 44.0 us; few tokens in fp32:
+// 8 x 43 x 2296, 591 blocks 716 -> 976 us).
+//
+// Parts are also the more exact form, since accumulators take fewer terms.  Relative error against float64 over 24
+// sizes of these ranges, whole -> parts: 1.3e-4 -> 2.6e-6 (bf16, 120000 features), 8.3e-6 -> 2.7e-7 (10000), 5 to 80
+// times less in bf16 and 2 to 6 times less in fp32, nowhere more.
 int plan_parts(GemmGeom& g, bool bf16, int sms) {
   const auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const int kb = bf16 ? tc::kBK : kSimtBK, kb_per_seg = (int)up(g.Kseg, kb);
@@ -100,7 +105,8 @@ int plan_parts(GemmGeom& g, bool bf16, int sms) {
   } else {
     const long long small = up(g.M, 64) * up(g.N, 64);
     whole = tiles * g.nz < sms ? fmax(0.9 * longest, 0.62 * total * small / sms) : 2.2 * longest;
-    split = parts * tiles < sms ? part * fmax(0.9, 0.62 * up(parts * small, sms)) : 2.2 * part * up(parts * tiles, slots);
+    split = parts * tiles < sms ? part * fmax(0.9, 0.62 * up(parts * small, sms))
+                                : 2.2 * part * up(parts * tiles, slots);
   }
   const double weights = (double)total * kb * g.N * (bf16 ? 2 : 4) / 5.5e6;
   split = fmax(split, weights) + 6.0 + 8.0 * parts * g.M * g.N / 5e6;
@@ -173,7 +179,8 @@ int clt_encoder_fwd_store(const void* xn, const void* W_enc, void* z_out, int B,
   Operand a{xn, 1, B, D, L}, b{W_enc, 0, F, D, L};
   epi::StoreZ<float>::Params p32{(float*)z_out};
   epi::StoreZ<bf16_t>::Params p16{(bf16_t*)z_out};
-  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, true>(g, a, b, p32, p16, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, true>(g, a, b, p32, p16, bf16, status,
+                                                                        (cudaStream_t)stream);
 }
 
 int clt_decoder_dense_fwd(const void* feat, const void* W_dec, const float* b_dec, float* recon, int B, int L, int D,
@@ -274,7 +281,8 @@ int clt_decoder_dense_bwd_dfeat_raw(const void* drecon, const void* W_dec, void*
   Operand a{drecon, 1, B, D, L}, b{W_dec, 1, F, D, P};
   epi::StoreZ<float>::Params p32{(float*)g_out};
   epi::StoreZ<bf16_t>::Params p16{(bf16_t*)g_out};
-  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, false>(g, a, b, p32, p16, bf16, status, (cudaStream_t)stream);
+  return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, false>(g, a, b, p32, p16, bf16, status,
+                                                                         (cudaStream_t)stream);
 }
 
 int clt_decoder_dense_bwd_dw(const void* feat, const void* drecon, float* dW, const float* rowcoef,

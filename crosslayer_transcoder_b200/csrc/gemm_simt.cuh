@@ -7,9 +7,10 @@
 // double-buffered: the global loads of the next tile are in flight, in registers, while the current one
 // is multiplied, and every load is 16 bytes along the operand's contiguous axis where its strides allow.
 // Each output is one fma chain in ascending k, whatever the tile.
-// 12-layer, 1024-feature, 512-token JumpReLU step (its five contractions): 12.6 -> 5.3 ms, 4.8 with the decoder in parts and the feature
-// gradient in half tiles; the kernel before gave a
-// thread one row x 64 columns, read K-contiguous operands 4 bytes a row, and loaded and multiplied in turn.
+// 12-layer, 1024-feature, 512-token JumpReLU step (its five contractions): 12.6 -> 5.3 ms, 4.8 with the decoder in
+// parts and the feature gradient in half tiles; the kernel before gave a thread one row x 64 columns, read K-contiguous
+// operands 4 bytes a row, and loaded and multiplied in turn.  At 8 x 8 the plain epilogue needs 126 registers; those of
+// the (Jump)ReLU spill around it (104 bytes forward, 812 backward, where half tiles spill none).
 //
 // The finished tile goes through shared memory, 64 columns at a time, into the shape that the
 // tcgen05 kernel reads out of tensor memory (a warp holds 32 rows, a lane 32 columns of its row), so

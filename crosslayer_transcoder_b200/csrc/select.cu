@@ -556,8 +556,8 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
   __syncwarp();
   // Trim when 64 (or k) entries have joined the k that are held, and before the next step could overflow the list: a
   // stale tau lets 4 values of a step join in the middle of a row of 32768, which costs more than a trim of 128
-  // (12 x 4000 rows of 32768, k = 32: 1.39 -> 1.15 ms; 12 x 2047 of 20000, k = 16: 0.51 -> 0.38 ms; trimming only when the list
-  // was full, always over 512 registers, before).
+  // (12 x 4000 rows of 32768, k = 32: 1.39 -> 1.15 ms; 12 x 2047 of 20000, k = 16: 0.51 -> 0.38 ms; trimming only when
+  // the list was full, always over 512 registers, before).
   const int trim_at = min(kStreamCap - 256, k + max(64, k));
   using CL = ChunkLoader<T>;
   // 256 columns per step (8 per lane); the next step's row values are requested before this step's are used

@@ -511,8 +511,12 @@ class StepEngine:
                            acc[2:4], b_cnt, L, D, s)
             all_reduce_sum(acc[0:4], group)             # encoder-side sums of all shards, loss sums of all owners
         else:
-            # bf16: whole chains whatever the batch.  Partial sums round differently, and in a small batch a
-            # (Jump)ReLU gradient can hang on one pre-activation that falls on the other side for it.
+            # bf16: whole chains whatever the batch, so that small steps give what they gave before there were
+            # parts.  That is not for exactness: the parts' sums are 5 to 80 times nearer to float64
+            # (csrc/gemm_dense.cu).  But the reconstruction's gradient is rounded to bf16, which turns the difference
+            # into one of 3e-4 to 5e-4 in the gradients (64 to 1000 tokens), and after two optimizer steps, which move
+            # a weight by the learning rate whatever the size of its gradient, into 3e-3 to 1.3e-2.  fp32 sums differ
+            # by 1e-6, inference feeds no gradient, and the auxiliary loss is a small share of its step's.
             self._decoder_dense_fwd(feat, W_op, dec.b.data if first_rank else None, recon, B, L, D, F, crosslayer, bf16,
                                     split=not bf16)
             if world > 1:
@@ -538,11 +542,14 @@ class StepEngine:
         """``(pre_actvs [B,L,F], features [B,L,F], recons_norm [B,L,D], recons [B,L,D])`` of
         ``CrossLayerTranscoder.forward`` (reference crosslayer_transcoder/model/clt.py:403-425) on this
         library's kernels from end to end: standardise + cast (``clt_prep_acts``), encoder contraction
-        (``clt_encoder_fwd_store``), the nonlinearity — (Jump)ReLU by ``clt_act_fwd``, PerLayerTopK by
+        (``clt_encoder_fwd_store``), the nonlinearity — (Jump)ReLU by ``clt_act_export``, PerLayerTopK by
         ``clt_select_topk``, BatchTopK / PerLayerBatchTopK by the histogram select, each exactly what the
         module's ``forward(..., layer="all")`` computes, running-threshold update included — the dense or
         sparse decoder, and the output de-standardisation (``clt_destandardize``).  The token-major fp32
-        tensors of the return value are written by ``clt_export_blf`` / ``clt_scatter_features``.  No
+        tensors of the return value are written by ``clt_act_export``, or ``clt_export_blf`` and
+        ``clt_scatter_features``.  The sparse decoder takes the CTA form of the gather at every size
+        (``module.decoder_gather_warp`` is a switch of the training step): the warp form took 358 us where it
+        takes 245 (1000 tokens, 12 layers, 16 entries of 768 columns).  No
         autograd graph is built.  On feature shards the partial reconstructions are summed over the ranks;
         the returned features are the rank's slice, and nonlinearities that rank across the whole feature
         axis (TopK, BatchTopK) are refused there."""
