@@ -57,9 +57,12 @@ def test_fp32_products(L, B, D, F):
 # few output tiles and long chains: parts of the contraction axis run side by side; the last shape stays whole
 @pytest.mark.parametrize("bf16", [0, 1])
 @pytest.mark.parametrize("L,B,D,F,cross", [(1, 257, 768, 30000, 0), (1, 1, 64, 4096, 0), (3, 65, 264, 2504, 1),
-                                           (5, 130, 64, 1368, 1), (2, 300, 320, 5000, 0), (12, 1000, 64, 512, 1)])
+                                           (5, 130, 64, 1368, 1), (2, 300, 320, 5000, 0), (12, 1000, 64, 512, 1),
+                                           (1, 300, 1024, 496, 0)])
 def test_split_decoder(L, B, D, F, cross, bf16):
     dev = "cuda:0"
+    parts = lib().query("clt_decoder_dense_parts", B, L, D, F, cross, bf16, 0)
+    assert (parts == 0) == (F == 496)
     g = torch.Generator(device=dev).manual_seed(F)
     P = L * (L + 1) // 2 if cross else L
     dt = torch.bfloat16 if bf16 else torch.float32
@@ -67,14 +70,16 @@ def test_split_decoder(L, B, D, F, cross, bf16):
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     whole, split, again = (torch.empty(B, L, D, device=dev) for _ in range(3))
     lib().call("clt_decoder_dense_fwd", feat, W, b, whole, B, L, D, F, cross, bf16, status, stream_ptr())
-    n = 600 * B * D
+    n = max(parts, 1) * B * D                               # as much as the library asks for, and no more
     for out in (split, again):
         ws = torch.full((n,), float("nan"), device=dev)     # every partial sum that is read was written
         lib().call("clt_decoder_dense_fwd_ws", feat, W, b, out, ws, n, B, L, D, F, cross, bf16, status, stream_ptr())
     assert torch.equal(split, again)
-    small = torch.empty_like(whole)
-    lib().call("clt_decoder_dense_fwd_ws", feat, W, b, small, ws, B * D - 1, B, L, D, F, cross, bf16, status, stream_ptr())
-    assert torch.equal(small, whole)                        # too little scratch: the unsplit chains
+    for less in (n - 1, B * D - 1):                         # too little scratch: the unsplit chains
+        small = torch.empty_like(whole)
+        lib().call("clt_decoder_dense_fwd_ws", feat, W, b, small, ws, less, B, L, D, F, cross, bf16, status, stream_ptr())
+        assert torch.equal(small, whole)
+    assert parts or torch.equal(split, whole)
     assert int(status) == 0
     for t in range(L):
         src = slice(0, t + 1) if cross else slice(t, t + 1)
