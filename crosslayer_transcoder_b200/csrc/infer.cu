@@ -168,13 +168,28 @@ int launch_act_export(const void* z, const float* bias, const float* theta, floa
   return 0;
 }
 
-// out[b, l, d] = recon[b, l, d] * sd[l, d] + mu[l, d]
-__global__ void destandardize_kernel(const float* __restrict__ recon, const float* __restrict__ mu,
-                                     const float* __restrict__ sd, float* __restrict__ out, long long total, int LD) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % LD);
-    out[i] = fmaf(recon[i], __ldg(sd + c), __ldg(mu + c));
+// out[b, l, d] = recon[b, l, d] * sd[l, d] + mu[l, d].  HBM-bound: blockIdx.x covers 256 V columns of the L D of a row,
+// blockIdx.y walks rows, so the statistics stay in registers and an element costs no 64-bit division (1000 x 12 x 768:
+// 33 -> 18 us, 4.1 TB/s; 1500 x 12 x 2304: 112 -> 64 us, 5.2 TB/s).  V = 4: 16-byte accesses.
+template <int V>
+__global__ void __launch_bounds__(256)
+destandardize_kernel(const float* __restrict__ recon, const float* __restrict__ mu, const float* __restrict__ sd,
+                     float* __restrict__ out, int B, long long LD) {
+  const long long c = (blockIdx.x * 256ll + threadIdx.x) * V;
+  if (c >= LD) return;
+  float m[V], d[V];
+#pragma unroll
+  for (int q = 0; q < V; ++q) m[q] = __ldg(mu + c + q), d[q] = __ldg(sd + c + q);
+#pragma unroll 4
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    const long long i = b * LD + c;
+    if constexpr (V == 4) {
+      const float4 r = *reinterpret_cast<const float4*>(recon + i);
+      *reinterpret_cast<float4*>(out + i) =
+          make_float4(fmaf(r.x, d[0], m[0]), fmaf(r.y, d[1], m[1]), fmaf(r.z, d[2], m[2]), fmaf(r.w, d[3], m[3]));
+    } else {
+      out[i] = fmaf(recon[i], d[0], m[0]);
+    }
   }
 }
 
@@ -249,8 +264,13 @@ int clt_import_rows(const float* src, int64_t ld, void* dst, int rows, int64_t K
 int clt_destandardize(const float* recon, const float* mu, const float* sd, float* out, int B, int L, int D,
                       clt_stream_t stream) {
   CLT_CHECK_ARG(recon && mu && sd && out && B > 0 && L > 0 && D > 0, "destandardize: bad arguments");
-  const long long total = (long long)B * L * D;
-  destandardize_kernel<<<grid_for(total), 256, 0, (cudaStream_t)stream>>>(recon, mu, sd, out, total, L * D);
+  const long long LD = (long long)L * D;
+  const int V = LD % 4 == 0 && ((uintptr_t)recon | (uintptr_t)out) % 16 == 0 ? 4 : 1;
+  const dim3 grid = row_grid(B, 1, LD, V);
+  if (V == 4)
+    destandardize_kernel<4><<<grid, 256, 0, (cudaStream_t)stream>>>(recon, mu, sd, out, B, LD);
+  else
+    destandardize_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(recon, mu, sd, out, B, LD);
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

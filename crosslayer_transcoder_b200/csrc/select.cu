@@ -449,6 +449,12 @@ select_topk_warp_kernel(const T* __restrict__ z, const float* __restrict__ b_enc
 // comes through L1, which the warps of the CTAs resident on an SM share because they walk the same
 // layer's bias at about the same pace.  The filter is one floating-point compare per element
 // (pre >= tau with tau > 0 also rejects everything that is not positive).  k <= kStreamCap - 256.
+//
+// kExport (inference): every pre-activation is written token-major on the way, and the token-major features, which are
+// zero but for the k selected.  Bound by the writes (4.7 to 5.8 TB/s in all) where the selection alone is bound by
+// instruction issue, so that the selection comes for free: rows of bf16 against the selection, the layout kernel, the zero
+// fill and the scatter, 12 x 1000 x 10000 (k = 16) 355 -> 256 us, 12 x 4000 x 32768 (k = 32) 3593 -> 2724 us; rows that
+// the two-sweep kernel selects from faster gain as well: 12 x 1000 x 4096 169 -> 123, x 1024 67 -> 59 us.
 // ---------------------------------------------------------------------------------------
 constexpr int kStreamWarps = 8;
 constexpr int kStreamMinF = 2048;   // shorter rows keep the one-warp-per-row two-sweep kernel
@@ -534,10 +540,11 @@ __device__ __forceinline__ unsigned stream_keep_top(float* cv, int* ci, int n, i
   return stream_keep_top_n<kStreamCap / 32>(cv, ci, n, k);
 }
 
-template <class T>
+template <class T, bool kExport>
 __global__ void __launch_bounds__(kStreamWarps * 32, 4)
 select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_enc, int* __restrict__ idx_out,
-                          float* __restrict__ val_out, unsigned* __restrict__ fired_bits, int B, int F, int k) {
+                          float* __restrict__ val_out, unsigned* __restrict__ fired_bits, float* __restrict__ pre_out,
+                          float* __restrict__ feat_out, int B, int F, int k) {
   __shared__ float c_val[kStreamWarps][kStreamCap];
   __shared__ int c_idx[kStreamWarps][kStreamCap];
   __shared__ int c_cnt[kStreamWarps];
@@ -548,6 +555,7 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
   const size_t row = (size_t)l * B + b;
   const T* zr = z + row * F;
   const float* br = b_enc + (size_t)l * F;  // read through L1: the 8 warps of a CTA walk the same layer's bias
+  const size_t out_row = kExport ? ((size_t)b * gridDim.y + l) * F : 0;
   float* cv = c_val[warp];
   int* ci = c_idx[warp];
   float tau = __uint_as_float(1u);          // smallest positive value: every positive value qualifies at first
@@ -575,6 +583,12 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
     CL::unpack(r, v);
     v[0] += c0.x, v[1] += c0.y, v[2] += c0.z, v[3] += c0.w;
     v[4] += c1.x, v[5] += c1.y, v[6] += c1.z, v[7] += c1.w;
+    if (kExport) {
+      if (i < F) {
+        st_f32x8(pre_out + out_row + i, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
+        st_f32x8(feat_out + out_row + i, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f));
+      }
+    }
     bool any = false;
 #pragma unroll
     for (int q = 0; q < 8; ++q) any |= v[q] >= tau;
@@ -655,6 +669,7 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
     const int f = live ? ci[j] : 0;
     io[j] = f;
     vo[j] = live ? cv[j] : 0.f;
+    if (kExport && live) feat_out[out_row + f] = cv[j];  // over the warp's zeros, which __syncwarp has put before it
     if (live && fired_bits != nullptr) atomicOr(fired_bits + (size_t)l * words + f / 32, 1u << (f & 31));
   }
 }
@@ -875,6 +890,15 @@ __global__ void topk_apply_threshold_kernel(int* __restrict__ idx, float* __rest
   for (int j = n_out + lane; j < k; j += 32) vr[j] = 0.f, ir[j] = 0;
 }
 
+template <class T, bool kExport>
+int launch_stream(const void* z, const float* b_enc, int* idx_out, float* val_out, unsigned* fired_bits, float* pre_out,
+                  float* feat_out, int B, int L, int F, int k, cudaStream_t s) {
+  select_topk_stream_kernel<T, kExport><<<dim3((B + kStreamWarps - 1) / kStreamWarps, L), kStreamWarps * 32, 0, s>>>(
+      (const T*)z, b_enc, idx_out, val_out, fired_bits, pre_out, feat_out, B, F, k);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
 }  // namespace
 
 }  // namespace clt
@@ -899,15 +923,8 @@ int clt_select_topk(const void* z, const float* b_enc, int* idx_out, float* val_
     // long rows: one streaming sweep per row.  Rows of up to 8192 columns (a feature shard's slice) stay with
     // the two-sweep warp kernel, whose second sweep comes from L2 and whose per-row bookkeeping is lighter:
     // 0.22 ms against 0.42 ms at 4096 columns, 0.36 against 0.67 ms at 8192 (12 layers x 4000 rows, k = 32)
-    dim3 grid((B + kStreamWarps - 1) / kStreamWarps, L);
-    if (bf16)
-      select_topk_stream_kernel<__nv_bfloat16><<<grid, kStreamWarps * 32, 0, s>>>(
-          (const __nv_bfloat16*)z, b_enc, idx_out, val_out, fired_bits, B, F, k);
-    else
-      select_topk_stream_kernel<float><<<grid, kStreamWarps * 32, 0, s>>>((const float*)z, b_enc, idx_out, val_out,
-                                                                          fired_bits, B, F, k);
-    CLT_CHECK_CUDA(cudaGetLastError());
-    return 0;
+    return bf16 ? launch_stream<__nv_bfloat16, false>(z, b_enc, idx_out, val_out, fired_bits, nullptr, nullptr, B, L, F, k, s)
+                : launch_stream<float, false>(z, b_enc, idx_out, val_out, fired_bits, nullptr, nullptr, B, L, F, k, s);
   }
   if (bf16) {
     if (warp_rows)
@@ -926,6 +943,22 @@ int clt_select_topk(const void* z, const float* b_enc, int* idx_out, float* val_
   }
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+
+int clt_select_topk_export(const void* z, const float* b_enc, int* idx_out, float* val_out, float* pre_out,
+                           float* features_out, int B, int L, int F, int k, int bf16, clt_stream_t stream) {
+  CLT_CHECK_ARG(B > 0 && L > 0 && L <= 65535 && F > 0 && F % 8 == 0, "select_topk_export: bad dims B=%d L=%d F=%d", B, L,
+                F);
+  CLT_CHECK_ARG(k > 0 && k <= F && k <= kStreamCap - 256, "select_topk_export: k=%d must be in [1, %d]", k,
+                kStreamCap - 256);
+  CLT_CHECK_ARG((long long)L * B < (1ll << 31), "select_topk_export: too many rows");
+  CLT_CHECK_ARG(z && b_enc && idx_out && val_out && pre_out && features_out, "select_topk_export: null pointer");
+  CLT_CHECK_ARG(((uintptr_t)z | (uintptr_t)b_enc) % 16 == 0 && aligned32(pre_out) && aligned32(features_out),
+                "select_topk_export: operands must be 16-byte, outputs 32-byte aligned");
+  return bf16 ? launch_stream<__nv_bfloat16, true>(z, b_enc, idx_out, val_out, nullptr, pre_out, features_out, B, L, F, k,
+                                                   (cudaStream_t)stream)
+              : launch_stream<float, true>(z, b_enc, idx_out, val_out, nullptr, pre_out, features_out, B, L, F, k,
+                                           (cudaStream_t)stream);
 }
 
 int clt_dead_compact(const uint8_t* dead, int* dead_list, int* n_dead, int L, int F, clt_stream_t stream) {

@@ -546,8 +546,8 @@ class StepEngine:
         ``clt_select_topk``, BatchTopK / PerLayerBatchTopK by the histogram select, each exactly what the
         module's ``forward(..., layer="all")`` computes, running-threshold update included — the dense or
         sparse decoder, and the output de-standardisation (``clt_destandardize``).  The token-major fp32
-        tensors of the return value are written by ``clt_act_export``, or ``clt_export_blf`` and
-        ``clt_scatter_features``.  The sparse decoder takes the CTA form of the gather at every size
+        tensors of the return value are written by ``clt_act_export`` or ``clt_select_topk_export``, else by
+        ``clt_export_blf`` and ``clt_scatter_features``.  The sparse decoder takes the CTA form of the gather at every size
         (``module.decoder_gather_warp`` is a switch of the training step): the warp form took 358 us where it
         takes 245 (1000 tokens, 12 layers, 16 entries of 768 columns).  No
         autograd graph is built.  On feature shards the partial reconstructions are summed over the ranks;
@@ -584,7 +584,10 @@ class StepEngine:
         z = torch.empty(L, B, F, dtype=T, device=dev)
         self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16), z, B, L, D, F, int(bf16), self.status, s)
         pre_actvs = torch.empty(B, L, F, dtype=torch.float32, device=dev)
-        if kind not in ("jumprelu", "relu"):
+        # TopK: the streaming selection writes both token-major results on its way, which saves a second sweep of z and
+        # a pass of zeros, at every row length that it takes (measurements at its kernel, csrc/select.cu)
+        one_sweep = kind == "topk" and F % 8 == 0 and 0 < int(nl.k) <= min(F, 256)
+        if kind not in ("jumprelu", "relu") and not one_sweep:
             self._call("clt_export_blf", z, enc.b.data, pre_actvs, B, L, F, int(bf16), s)
         features = torch.empty(B, L, F, dtype=torch.float32, device=dev)
         recon = torch.empty(B, L, D, dtype=torch.float32, device=dev)
@@ -609,8 +612,12 @@ class StepEngine:
             else:
                 idx = torch.empty(L, B, k, dtype=torch.int32, device=dev)
                 val = torch.empty(L, B, k, dtype=torch.float32, device=dev)
-                self._call("clt_select_topk", z, enc.b.data, idx, val, None, B, L, F, k, int(bf16), s)
-                self._call("clt_scatter_features", idx, val, None, features, B, L, F, k, B * k, self.status, s)
+                if one_sweep:
+                    self._call("clt_select_topk_export", z, enc.b.data, idx, val, pre_actvs, features, B, L, F, k,
+                               int(bf16), s)
+                else:
+                    self._call("clt_select_topk", z, enc.b.data, idx, val, None, B, L, F, k, int(bf16), s)
+                    self._call("clt_scatter_features", idx, val, None, features, B, L, F, k, B * k, self.status, s)
                 self._call("clt_sparse_decoder_fwd", idx, val, None, None, B * k, W_op, bias, recon, B, L, D, F, k,
                            crosslayer, 0, int(bf16), self.status, s)
         else:

@@ -178,6 +178,12 @@ int clt_dead_update(int64_t* last_active, uint32_t* fired_bits, uint8_t* dead, i
 int clt_select_topk(const void* z, const float* b_enc, int* idx_out, float* val_out, uint32_t* fired_bits,
                     int B, int L, int F, int k, int bf16, clt_stream_t stream);
 
+/* clt_select_topk, clt_export_blf and clt_scatter_features of the inference forward in one sweep of z: pre_out [B,L,F] =
+ * z + b_enc, features_out [B,L,F] = the selected values, 0 elsewhere (both fp32, 32-byte aligned).  F a multiple of 8,
+ * 1 <= k <= 256; the entries of a row come largest value first. */
+int clt_select_topk_export(const void* z, const float* b_enc, int* idx_out, float* val_out, float* pre_out,
+                           float* features_out, int B, int L, int F, int k, int bf16, clt_stream_t stream);
+
 /* Ascending list of the dead features of every layer: dead_list [L, F], n_dead [L]
  * (idxs_dead of clt_lightning.py:286, compacted). */
 int clt_dead_compact(const uint8_t* dead, int* dead_list, int* n_dead, int L, int F, clt_stream_t stream);
