@@ -1032,4 +1032,50 @@ int finalize_loss(const float* mse_acc, const float* enc_acc, float* loss, float
   return 0;
 }
 
+// out[j, i] = float(stat j [i]) for the four statistics of the standardizers
+template <class T>
+__global__ void cast_stats_kernel(const T* a, const T* b, const T* c, const T* d, float* __restrict__ out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const T* const src[4] = {a, b, c, d};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) out[(long long)j * n + i] = (float)src[j][i];
+}
+int cast_stats(const void* a, const void* b, const void* c, const void* d, int dtype, float* out, int n,
+               cudaStream_t s) {
+  const int blocks = (n + 255) / 256;
+  if (dtype == 1)
+    cast_stats_kernel<__half><<<blocks, 256, 0, s>>>((const __half*)a, (const __half*)b, (const __half*)c,
+                                                     (const __half*)d, out, n);
+  else
+    cast_stats_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
+                                                            (const __nv_bfloat16*)c, (const __nv_bfloat16*)d, out, n);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// blockIdx.y picks one of four arrays; what a step's atomics add to is small, so one launch counts, not its rate
+struct ZeroArrays {
+  float* p[4];
+  long long n[4];
+};
+__global__ void __launch_bounds__(256) zero4_kernel(ZeroArrays z) {
+  float* p = z.p[blockIdx.y];
+  const long long n = z.n[blockIdx.y];
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll) p[i] = 0.f;
+}
+int zero4(float* const (&p)[4], const long long (&n)[4], cudaStream_t s) {
+  ZeroArrays z;
+  long long most = 0;
+  for (int j = 0; j < 4; ++j) {
+    z.p[j] = p[j], z.n[j] = p[j] != nullptr && n[j] > 0 ? n[j] : 0;
+    most = z.n[j] > most ? z.n[j] : most;
+  }
+  if (most == 0) return 0;
+  const long long want = (most + 255) / 256;
+  zero4_kernel<<<dim3((unsigned)(want < 148 * 8 ? want : 148 * 8), 4), 256, 0, s>>>(z);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
 }  // namespace clt

@@ -117,6 +117,18 @@ int clt_loss_bwd(const float* recon, const float* aux, const void* batch, int in
                   (cudaStream_t)stream);
 }
 
+int clt_cast_stats(const void* a, const void* b, const void* c, const void* d, int dtype, float* out, int n,
+                   clt_stream_t stream) {
+  CLT_CHECK_ARG(a && b && c && d && out && n > 0, "cast_stats: null pointer or no values");
+  CLT_CHECK_ARG(dtype == 1 || dtype == 2, "cast_stats: dtype %d is not a 16-bit one", dtype);
+  return cast_stats(a, b, c, d, dtype, out, n, (cudaStream_t)stream);
+}
+
+int clt_zero4(float* p0, int64_t n0, float* p1, int64_t n1, float* p2, int64_t n2, float* p3, int64_t n3,
+              clt_stream_t stream) {
+  return zero4({p0, p1, p2, p3}, {(long long)n0, (long long)n1, (long long)n2, (long long)n3}, (cudaStream_t)stream);
+}
+
 int clt_sum_slots(const void* slots, float* out, int n_slots, int64_t n, int slots_bf16, clt_stream_t stream) {
   CLT_CHECK_ARG(slots && out && n_slots > 0 && n >= 0 && n % (slots_bf16 ? 8 : 4) == 0,
                 "sum_slots: bad arguments (n must be a multiple of 4, of 8 for bf16 slots)");

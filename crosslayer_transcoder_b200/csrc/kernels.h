@@ -32,6 +32,8 @@ int dead_update(long long* last_active, unsigned* fired_bits, unsigned char* dea
 int adam_step(float* p, const float* g, float* m, float* v, void* shadow_bf16, long long n, float lr, float beta1,
               float beta2, float eps, float weight_decay, int decoupled, long long step, int num_sms, cudaStream_t s);
 int cast_bf16(const float* src, void* dst, long long n, cudaStream_t s);
+int cast_stats(const void* a, const void* b, const void* c, const void* d, int dtype, float* out, int n, cudaStream_t s);
+int zero4(float* const (&p)[4], const long long (&n)[4], cudaStream_t s);
 int finalize_loss(const float* mse_acc, const float* enc_acc, float* loss, float* terms, float inv_bld, float lam_over_b,
                   float pal_over_bl, float aux_scale, cudaStream_t s);
 

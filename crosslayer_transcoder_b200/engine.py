@@ -58,6 +58,10 @@ class FlatParams:
         self._bytes = [4 * self.offsets[id(p)] for p in self.params]
         self._shadow_version = None
         self._operands: Dict[int, torch.Tensor] = {}
+        # views of this object's own buffers, made once: a slice and a view cost 5 us, a step used two dozen
+        self._grads: Dict[int, torch.Tensor] = {}
+        self._decoder: Dict[bool, tuple] = {}
+        self._strided = [(p.shape, p.data.stride(), self.offsets[id(p)]) for p in self.params]
         if want_bf16:
             self.ensure_shadow()
 
@@ -66,6 +70,14 @@ class FlatParams:
         v = self._operands.get(id(p))
         if v is None:
             v = self._operands[id(p)] = self.view_of(p, self.shadow)
+        return v
+
+    def grad_of(self, p: torch.nn.Parameter) -> torch.Tensor:
+        """``p``'s slice of the flat gradient, for the kernels (never handed to autograd, which keeps a gradient as
+        ``.grad`` without copying it only when nothing else holds the tensor)."""
+        v = self._grads.get(id(p))
+        if v is None:
+            v = self._grads[id(p)] = self.view_of(p, self.grad)
         return v
 
     def view_of(self, p: torch.nn.Parameter, buf: torch.Tensor) -> torch.Tensor:
@@ -88,6 +100,7 @@ class FlatParams:
         if self.shadow is None:
             self.shadow = torch.empty(self.numel, dtype=torch.bfloat16, device=self.device)
             self._operands.clear()
+            self._decoder.clear()
             self._shadow_version = None
         if self._shadow_version != v:
             lib().call("clt_cast_bf16", self.flat, self.shadow, self.numel, stream_ptr())
@@ -124,6 +137,8 @@ class StepEngine:
         self.launches = 0                         # kernels launched by this engine (for reporting)
         self.last_terms: Optional[torch.Tensor] = None
         self.profile: Optional[dict] = None
+        self._library = None
+        self._sum_views: Dict[str, tuple] = {}    # see _sums
         # the device status word is copied to pinned host memory after every backward and looked at,
         # without waiting, when the next steps begin
         self.optimizer = None                     # the FusedAdam of configure_optimizers (for fuse_optimizer)
@@ -143,7 +158,7 @@ class StepEngine:
         dict, CUDA events around the call collect per-entry-point device time (``tag`` keeps apart two uses
         of one entry point with different shapes)."""
         if self.profile is None:
-            lib().call(name, *args)
+            (self._library or self._bind()).call(name, *args)
         else:
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
@@ -151,6 +166,10 @@ class StepEngine:
             e1.record()
             self.profile.setdefault(name + tag, []).append((e0, e1))
         self.launches += 1
+
+    def _bind(self):
+        self._library = lib()
+        return self._library
 
     def profile_summary(self) -> Dict[str, dict]:
         """{entry point: {"launches", "ms_total", "ms_avg"}} from the collected events (synchronises)."""
@@ -210,10 +229,11 @@ class StepEngine:
             return
         if self._status_host is None:
             self._status_host = torch.zeros(2, dtype=torch.int32).pin_memory()
+            self._status_slots = self._status_host[0:1], self._status_host[1:2]
             self._status_evt = [torch.cuda.Event(), torch.cuda.Event()]
         slot = self._status_slot
         self._status_slot ^= 1
-        self._status_host[slot:slot + 1].copy_(self.status, non_blocking=True)
+        self._status_slots[slot].copy_(self.status, non_blocking=True)
         self._status_evt[slot].record()
         self._status_pending[slot] = True
 
@@ -240,6 +260,9 @@ class StepEngine:
     def _dec_flat(self, bf16: bool):
         """(operand buffer [P,F,D], fp32 master [P,F,D], gradient [P,F,D]) of the decoder blocks;
         they are adjacent in the flat buffer in block order."""
+        cached = self.flat._decoder.get(bf16)
+        if cached is not None:
+            return cached
         dec = self.module.model.decoder
         blocks = dec.blocks()
         F, D = dec.d_features, dec.d_acts
@@ -254,7 +277,9 @@ class StepEngine:
         P = n // (F * D)
         sl = slice(o0, o0 + n)
         op = (self.flat.shadow if bf16 else self.flat.flat)[sl].view(P, F, D)
-        return op, self.flat.flat[sl].view(P, F, D), self.flat.grad[sl].view(P, F, D)
+        views = op, self.flat.flat[sl].view(P, F, D), self.flat.grad[sl].view(P, F, D)
+        self.flat._decoder[bf16] = views
+        return views
 
     def _stats(self):
         m = self.module.model
@@ -263,8 +288,17 @@ class StepEngine:
             raise CltError("the fused step needs both standardizers")
         if not (ins.is_initialized and outs.is_initialized):
             raise ValueError("Standardizer not initialized")
+        stats = ins.mean, ins.std, outs.mean, outs.std
+        t0 = stats[0]
+        if t0.dtype in (torch.float16, torch.bfloat16) and \
+                all(t.dtype == t0.dtype and t.shape == t0.shape and t.device == t0.device and t.is_cuda and
+                    t.is_contiguous() for t in stats):
+            # statistics of a 16-bit batch: one launch instead of four conversions
+            out = torch.empty(4, *t0.shape, dtype=torch.float32, device=t0.device)
+            self._call("clt_cast_stats", *stats, DTYPE_CODE[t0.dtype], out, t0.numel(), stream_ptr())
+            return out.unbind(0)
         f = lambda t: t if t.dtype == torch.float32 and t.is_contiguous() else t.detach().float().contiguous()
-        return f(ins.mean), f(ins.std), f(outs.mean), f(outs.std)
+        return tuple(f(t) for t in stats)
 
     def _fuse_activation(self, D: int, F: int, bf16: bool) -> bool:
         """Fuse the (Jump)ReLU into the contraction epilogues?  ``module.fuse_activation`` forces it
@@ -426,6 +460,22 @@ class StepEngine:
 
         all_reduce_sum(px["token"], self.module.tp_group)
 
+    @staticmethod
+    def _new_loss(dev):
+        """(loss scalar, its four summands): tensors of this step's own."""
+        return torch.empty((), dtype=torch.float32, device=dev), torch.empty(4, dtype=torch.float32, device=dev)
+
+    def _sums(self, name: str, n: int, parts: int, shape, dev):
+        """Reconstruction buffer ``name`` of ``parts`` x ``n`` floats with a tail of 8 loss sums, in one allocation that
+        feature shards reduce together: (whole, [the parts as ``shape``], tail, tail[0:2], tail[2:4])."""
+        buf = self.ws.get(name, (parts * n + 8,), torch.float32, dev)
+        views = self._sum_views.get(name)
+        if views is None or views[0] is not buf or views[1][0].shape != shape:
+            acc = buf[parts * n:]
+            views = self._sum_views[name] = (buf, [buf[i * n:(i + 1) * n].view(shape) for i in range(parts)], acc,
+                                             acc[0:2], acc[2:4])
+        return views
+
     # ------------------------------------------------------------------ forward
     def forward(self, batch: torch.Tensor, hyper: dict) -> torch.Tensor:
         """Run the forward half of the step on ``batch`` ``[B, 2, L, D]`` and return the scalar
@@ -447,7 +497,7 @@ class StepEngine:
             ctx = self._forward_batchtopk(batch, hyper, bf16)
         else:
             raise NotImplementedError(f"nonlinearity kind {kind!r}")
-        self.last_terms = ctx["out"][1:5]          # mse, sparsity, pre-activation, auxiliary summands
+        self.last_terms = ctx["terms"]             # mse, sparsity, pre-activation, auxiliary summands
         self._last_ctx = ctx
         params = self.flat.params
         return _StepFunction.apply(self, ctx, *params)
@@ -468,9 +518,8 @@ class StepEngine:
         feat = ws.get("feat", (L, B, F), T, dev)
         # reconstruction buffer with an 8-float tail: [0:2] encoder-side loss sums (summed over
         # feature shards together with the partial reconstructions), [2:4] reconstruction-loss sums
-        rbuf = ws.get("recon", (B * L * D + 8,), torch.float32, dev)
-        recon, acc = rbuf[: B * L * D].view(B, L, D), rbuf[B * L * D:]
-        out = torch.empty(5, dtype=torch.float32, device=dev)       # loss + 4 terms
+        rbuf, (recon,), acc, acc_enc, acc_rec = self._sums("recon", B * L * D, 1, (B, L, D), dev)
+        loss, terms = self._new_loss(dev)
         acc.zero_()
         world, group = getattr(mod, "tp_world", 1), getattr(mod, "tp_group", None)
         first_rank = getattr(mod, "tp_rank", 0) == 0
@@ -488,10 +537,10 @@ class StepEngine:
         fused = self._fuse_activation(D, F, bf16)
         if fused:
             self._call("clt_encoder_fwd_act", xn, self._operand(enc.W, bf16), enc.b.data, theta, norm, z, feat,
-                       self.fired, acc[0:2], c_sp, use_tanh, want_pre, B, L, D, F, int(bf16), self.status, s)
+                       self.fired, acc_enc, c_sp, use_tanh, want_pre, B, L, D, F, int(bf16), self.status, s)
         else:
             self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16), z, B, L, D, F, int(bf16), self.status, s)
-            self._call("clt_act_fwd", z, enc.b.data, theta, norm, feat, self.fired, acc[0:2], c_sp, use_tanh, want_pre,
+            self._call("clt_act_fwd", z, enc.b.data, theta, norm, feat, self.fired, acc_enc, c_sp, use_tanh, want_pre,
                        B, L, F, int(bf16), s)
         px = None
         if world > 1 and getattr(mod, "tp_fused", False) and D % 8 == 0:
@@ -508,7 +557,7 @@ class StepEngine:
             b_lo, b_cnt = px["b_lo"], px["b_cnt"]
             if b_cnt > 0:
                 self._call("clt_loss_fwd", px["recon_own"], None, batch[b_lo:b_lo + b_cnt], in_code, mu_o, sd_o,
-                           acc[2:4], b_cnt, L, D, s)
+                           acc_rec, b_cnt, L, D, s)
             all_reduce_sum(acc[0:4], group)             # encoder-side sums of all shards, loss sums of all owners
         else:
             # bf16: whole chains whatever the batch, so that small steps give what they gave before there were
@@ -523,15 +572,15 @@ class StepEngine:
                 from .parallel import all_reduce_sum
 
                 all_reduce_sum(rbuf[: B * L * D + 2], group)      # partial reconstructions + encoder-side sums
-            self._call("clt_loss_fwd", recon, None, batch, in_code, mu_o, sd_o, acc[2:4], B, L, D, s)
+            self._call("clt_loss_fwd", recon, None, batch, in_code, mu_o, sd_o, acc_rec, B, L, D, s)
         pal = float(h.get("pre_actv_loss", 0.0))
-        self._call("clt_finalize_loss", acc[2:4], acc[0:2], out[0:1], out[1:5], 1.0 / (B * L * D), lam / B,
+        self._call("clt_finalize_loss", acc_rec, acc_enc, loss, terms, 1.0 / (B * L * D), lam / B,
                    pal / (B * L), 0.0, s)
         self._call("clt_dead_update", mod.last_active, self.fired, None, B, int(mod.tokens_till_dead), L, F,
                    self._dead_count(dev), None, s)
         return dict(kind=h["kind"], bf16=bf16, batch=batch, B=B, L=L, D=D, F=F, crosslayer=crosslayer, lam=lam,
                     pal=pal, c=float(h.get("c_sparsity", 1.0)), use_tanh=int(h.get("use_tanh", True)),
-                    bandwidth=self._bandwidth(nl) if h["kind"] == "jumprelu" else 1.0, out=out,
+                    bandwidth=self._bandwidth(nl) if h["kind"] == "jumprelu" else 1.0, loss=loss, terms=terms,
                     stats=(mu_i, sd_i, mu_o, sd_o), norm=norm, in_code=in_code, fused=fused, px=px,
                     recon_rows=(px["recon_own"], px["b_lo"], px["b_cnt"]) if px is not None else (recon, 0, B),
                     l0_src=(feat, 2 if bf16 else 0, B * F))
@@ -709,14 +758,18 @@ class StepEngine:
             self.after_backward()
         self.post_status()
 
-    def _zero_small_grads(self):
-        """Gradients accumulated with atomics start from zero; contraction outputs are overwritten."""
-        model = self.module.model
-        small = [model.encoder.b, model.decoder.b]
-        if hasattr(model.nonlinearity, "theta"):
-            small.append(model.nonlinearity.theta)
-        for p in small:
-            self.flat.view_of(p, self.flat.grad).zero_()
+    def _zero(self, *tensors):
+        """Up to four fp32 tensors (or None) are set to zero by one launch: what is accumulated with atomics starts so."""
+        args = []
+        for t in tensors + (None,) * (4 - len(tensors)):
+            args += (t, t.numel() if t is not None else 0)
+        self._call("clt_zero4", *args, stream_ptr())
+
+    @staticmethod
+    def _loss_scale(gscale: torch.Tensor) -> torch.Tensor:
+        """The loss gradient as a device float."""
+        return gscale if gscale.dtype == torch.float32 and gscale.numel() == 1 else \
+            gscale.detach().to(torch.float32).reshape(1).contiguous()
 
     def _backward_dense(self, c, gscale):
         model = self.module.model
@@ -727,14 +780,16 @@ class StepEngine:
         s = stream_ptr()
         ws = self.ws
         xn, z, feat = ws.buf["xn"], ws.buf["z"], ws.buf["feat"]
-        recon = ws.buf["recon"][: B * L * D].view(B, L, D)
+        _, (recon,), *_ = self._sums("recon", B * L * D, 1, (B, L, D), dev)
         drecon = ws.get("drecon", (L, B, D), T, dev)
         dpre = ws.get("dpre", (L, B, F), T, dev)
         _, _, mu_o, sd_o = c["stats"]
-        g = self.flat.grad
-        gview = lambda p: self.flat.view_of(p, g)
-        self._zero_small_grads()
-        gs = gscale.detach().to(torch.float32).reshape(1).contiguous()
+        gview = self.flat.grad_of
+        norm = c["norm"]
+        dnorm = ws.get("dnorm", (L, F), torch.float32, dev) if norm is not None else None
+        # gradients that are accumulated with atomics; contraction outputs are overwritten
+        self._zero(gview(enc.b), gview(dec.b), gview(nl.theta) if hasattr(nl, "theta") else None, dnorm)
+        gs = self._loss_scale(gscale)
         px = c.get("px")
         if px is not None:
             from .parallel import all_reduce_sum
@@ -753,11 +808,6 @@ class StepEngine:
         W_op, W_master, dW_dec = self._dec_flat(bf16)
         theta = nl.theta.data if c["kind"] == "jumprelu" else None
         dtheta = gview(nl.theta) if c["kind"] == "jumprelu" else None
-        norm = c["norm"]
-        dnorm = None
-        if norm is not None:
-            dnorm = ws.get("dnorm", (L, F), torch.float32, dev)
-            dnorm.zero_()
         if c["fused"]:
             self._call("clt_decoder_dense_bwd_dfeat", drecon, W_op, z, enc.b.data, theta, norm, dpre, dtheta,
                        gview(enc.b), dnorm, c["bandwidth"], c["lam"] / B, c["c"], c["pal"] / (B * L), c["use_tanh"], gs,
@@ -801,9 +851,8 @@ class StepEngine:
         # [reconstruction | auxiliary reconstruction | 8-float tail of loss sums]: the first two are
         # partial sums over this rank's features and are reduced together across feature shards
         n_rec = B * L * D
-        rbuf = ws.get("recon2", (2 * n_rec + 8,), torch.float32, dev)
-        recon, aux_recon_buf, acc = rbuf[:n_rec].view(B, L, D), rbuf[n_rec:2 * n_rec].view(B, L, D), rbuf[2 * n_rec:]
-        out = torch.empty(5, dtype=torch.float32, device=dev)
+        rbuf, (recon, aux_recon_buf), acc, _, acc_rec = self._sums("recon2", n_rec, 2, (B, L, D), dev)
+        loss, terms = self._new_loss(dev)
         acc.zero_()
         world, group = getattr(mod, "tp_world", 1), getattr(mod, "tp_group", None)
         bias = dec.b.data if getattr(mod, "tp_rank", 0) == 0 else None      # added once, not per shard
@@ -947,16 +996,16 @@ class StepEngine:
             b_lo, b_cnt = px["b_lo"], px["b_cnt"]
             if b_cnt > 0:
                 self._call("clt_loss_fwd", px["recon_own"], px["aux_own"] if aux is not None else None,
-                           batch[b_lo:b_lo + b_cnt], in_code, mu_o, sd_o, acc[2:4], b_cnt, L, D, s)
-            all_reduce_sum(acc[2:4], group)             # loss sums of all owners
+                           batch[b_lo:b_lo + b_cnt], in_code, mu_o, sd_o, acc_rec, b_cnt, L, D, s)
+            all_reduce_sum(acc_rec, group)             # loss sums of all owners
         else:
             for h_ in pending:
                 h_.wait()
-            self._call("clt_loss_fwd", recon, aux_recon, batch, in_code, mu_o, sd_o, acc[2:4], B, L, D, s)
-        self._call("clt_finalize_loss", acc[2:4], None, out[0:1], out[1:5], 1.0 / (B * L * D), 0.0, 0.0,
+            self._call("clt_loss_fwd", recon, aux_recon, batch, in_code, mu_o, sd_o, acc_rec, B, L, D, s)
+        self._call("clt_finalize_loss", acc_rec, None, loss, terms, 1.0 / (B * L * D), 0.0, 0.0,
                    aux_scale if aux is not None else 0.0, s)
-        return dict(kind="topk", bf16=bf16, batch=batch, B=B, L=L, D=D, F=F, k=kk, crosslayer=crosslayer, out=out,
-                    stats=(mu_i, sd_i, mu_o, sd_o), in_code=in_code, aux=aux, aux_scale=aux_scale, idx=idx, val=val,
+        return dict(kind="topk", bf16=bf16, batch=batch, B=B, L=L, D=D, F=F, k=kk, crosslayer=crosslayer,
+                    loss=loss, terms=terms, stats=(mu_i, sd_i, mu_o, sd_o), in_code=in_code, aux=aux, aux_scale=aux_scale, idx=idx, val=val,
                     px=px,
                     recon_rows=(px["recon_own"], px["b_lo"], px["b_cnt"]) if px is not None else (recon, 0, B),
                     l0_src=(val, 0, B * kk))
@@ -986,9 +1035,8 @@ class StepEngine:
         xn = ws.get("xn", (L, B, D), T, dev)
         z = ws.get("z", (L, B, F), T, dev)
         n_rec = B * L * D
-        rbuf = ws.get("recon2", (2 * n_rec + 8,), torch.float32, dev)
-        recon, acc = rbuf[:n_rec].view(B, L, D), rbuf[2 * n_rec:]
-        out = torch.empty(5, dtype=torch.float32, device=dev)
+        rbuf, (recon, _), acc, _, acc_rec = self._sums("recon2", n_rec, 2, (B, L, D), dev)
+        loss, terms = self._new_loss(dev)
         acc.zero_()
         in_code = DTYPE_CODE[batch.dtype]
         W_op, _, _ = self._dec_flat(bf16)
@@ -1013,8 +1061,8 @@ class StepEngine:
             b_lo, b_cnt = px["b_lo"], px["b_cnt"]
             if b_cnt > 0:
                 self._call("clt_loss_fwd", px["recon_own"], None, batch[b_lo:b_lo + b_cnt], in_code, mu_o, sd_o,
-                           acc[2:4], b_cnt, L, D, s)
-            all_reduce_sum(acc[2:4], group)             # loss sums of all owners
+                           acc_rec, b_cnt, L, D, s)
+            all_reduce_sum(acc_rec, group)             # loss sums of all owners
         else:
             self._call("clt_sparse_decoder_fwd", idx, val, row_start, row_cnt, npl, W_op, bias, recon, B, L, D, F, 1,
                        crosslayer, self._gather_form(k, world, D), int(bf16), self.status, s)
@@ -1022,10 +1070,10 @@ class StepEngine:
                 from .parallel import all_reduce_sum
 
                 all_reduce_sum(rbuf[:n_rec], group)
-            self._call("clt_loss_fwd", recon, None, batch, in_code, mu_o, sd_o, acc[2:4], B, L, D, s)
-        self._call("clt_finalize_loss", acc[2:4], None, out[0:1], out[1:5], 1.0 / (B * L * D), 0.0, 0.0, 0.0, s)
-        return dict(kind="batchtopk", bf16=bf16, batch=batch, B=B, L=L, D=D, F=F, k=1, crosslayer=crosslayer, out=out,
-                    stats=(mu_i, sd_i, mu_o, sd_o), in_code=in_code, aux=None, aux_scale=0.0, idx=idx, val=val,
+            self._call("clt_loss_fwd", recon, None, batch, in_code, mu_o, sd_o, acc_rec, B, L, D, s)
+        self._call("clt_finalize_loss", acc_rec, None, loss, terms, 1.0 / (B * L * D), 0.0, 0.0, 0.0, s)
+        return dict(kind="batchtopk", bf16=bf16, batch=batch, B=B, L=L, D=D, F=F, k=1, crosslayer=crosslayer,
+                    loss=loss, terms=terms, stats=(mu_i, sd_i, mu_o, sd_o), in_code=in_code, aux=None, aux_scale=0.0, idx=idx, val=val,
                     npl=npl, etok=etok, px=px,
                     recon_rows=(px["recon_own"], px["b_lo"], px["b_cnt"]) if px is not None else (recon, 0, B),
                     l0_src=(val, 0, npl))
@@ -1119,16 +1167,15 @@ class StepEngine:
         ws = self.ws
         xn = ws.buf["xn"]
         n_rec = B * L * D
-        recon = ws.buf["recon2"][:n_rec].view(B, L, D)
-        aux_recon = ws.buf["recon2"][n_rec:2 * n_rec].view(B, L, D)
+        _, (recon, aux_recon), *_ = self._sums("recon2", n_rec, 2, (B, L, D), dev)
         aux = c["aux"]
         drecon = ws.get("drecon", (L, B, D), T, dev)
         daux = ws.get("daux", (L, B, D), T, dev) if aux is not None else None
         _, _, mu_o, sd_o = c["stats"]
-        g = self.flat.grad
-        gview = lambda p: self.flat.view_of(p, g)
-        gview(dec.b).zero_()
-        gs = gscale.detach().to(torch.float32).reshape(1).contiguous()
+        gview = self.flat.grad_of
+        db_c = ws.get("db_c", (L, aux["nd_pad"]), torch.float32, dev) if aux is not None else None
+        self._zero(gview(dec.b), db_c)
+        gs = self._loss_scale(gscale)
         px = c.get("px")
         if px is not None:
             # owned rows only; the gradient rows go straight into every rank's buffers, and the all-reduce
@@ -1159,7 +1206,7 @@ class StepEngine:
         dval = ws.get("dval", (L, npl), torch.float32, dev)
         self._call("clt_csc_build", idx, val, col_ptr, cursor, ent, npl, L, F, self.status, s)
         fuse_opt = self._fused_optimizer(F)
-        dW_c = dpre_c = db_c = dead_pos = None
+        dW_c = dpre_c = dead_pos = None
         if aux is not None:
             # position of every dead feature in the compact operands: the feature-major kernels below add the
             # auxiliary loss's compact gradients through it
@@ -1172,8 +1219,6 @@ class StepEngine:
             P = w_c.shape[0]
             zeros_b = ws.get("zeros_b", (L, nd_pad), torch.float32, dev, zero=True)
             dpre_c = ws.get("dpre_c", (L, B, nd_pad), T, dev)
-            db_c = ws.get("db_c", (L, nd_pad), torch.float32, dev)
-            db_c.zero_()
             # gradient w.r.t. the auxiliary features, ReLU-masked by the selection (a_aux > 0)
             self._call("clt_decoder_dense_bwd_dfeat", daux, w_c, a_aux, zeros_b, None, None, dpre_c, None, db_c, None,
                        1.0, 0.0, 1.0, 0.0, 0, None, B, L, D, nd_pad, cross, int(bf16), self.status, s)
@@ -1216,7 +1261,7 @@ class StepEngine:
     def _aux_state(self):
         st = getattr(self, "_aux_hist", None)
         if st is None:
-            st = self._aux_hist = dict(step=0, host=torch.zeros(2, 2, dtype=torch.int32).pin_memory(),
+            st = self._aux_hist = dict(step=0, host=torch.zeros(2, 2, dtype=torch.int32).pin_memory(), soon=None,
                                        evt=[torch.cuda.Event(), torch.cuda.Event()])
         return st
 
@@ -1235,7 +1280,7 @@ class StepEngine:
             nd = int(n_dead.max())                              # blocking: first two steps only
         else:
             st["evt"][i & 1].synchronize()                      # the copy made two steps ago into this slot
-            nd = int(st["host"][i & 1, 0])
+            nd = int(st["soon"][i & 1].max())
         return max(64, _round_up(nd, 64))
 
     def _aux_exchange(self, soon_dead: torch.Tensor, cnt, k_aux: int) -> bool:
@@ -1249,16 +1294,18 @@ class StepEngine:
         i = st["step"]
         st["step"] = i + 1
         slot = i & 1
+        if st["soon"] is None:      # two rows of pinned memory, per-layer counts of the even and the odd steps
+            st["soon"] = torch.zeros(2, soon_dead.numel(), dtype=torch.int32).pin_memory().unbind(0)
+        st["soon"][slot].copy_(soon_dead, non_blocking=True)
         if cnt is None:
             exchange = False
-            st["host"][slot, 0].copy_(soon_dead.max(), non_blocking=True)
         else:
             cmax_t = cnt.max()
             if i < 2:
                 exchange = int(cmax_t) > k_aux                   # blocking: first two steps only
             else:
                 exchange = 4 * int(st["host"][slot, 1]) > 3 * k_aux
-            st["host"][slot].copy_(torch.stack([soon_dead.max(), cmax_t]).to(torch.int32), non_blocking=True)
+            st["host"][slot, 1].copy_(cmax_t.to(torch.int32), non_blocking=True)
         st["evt"][slot].record()
         return exchange
 
@@ -1296,7 +1343,7 @@ class _StepFunction(torch.autograd.Function):
     def forward(ctx, engine: StepEngine, step_ctx: dict, *params):
         ctx.engine, ctx.step_ctx = engine, step_ctx
         ctx.n = len(params)
-        return step_ctx["out"][0].clone()
+        return step_ctx.pop("loss")     # a tensor of this step's own; kept in the context it would keep itself alive
 
     @staticmethod
     def backward(ctx, grad_out):
@@ -1315,13 +1362,13 @@ class _StepFunction(torch.autograd.Function):
         if getattr(eng, "decoder_updated", False):
             updated = {id(w) for w in eng.module.model.decoder.blocks()}
         grads = []
-        for p, al in zip(fp.params, aliased):
-            gv = fp.view_of(p, fp.grad)
+        for p, al, (shape, stride, offset) in zip(fp.params, aliased, fp._strided):
             if id(p) in updated:
                 grads.append(None)             # already stepped by the fused decoder backward
             elif al:
                 grads.append(fp.view_of(p, saved))
             else:
+                gv = fp.grad.as_strided(shape, stride, offset)      # view_of in one operation
                 # a gradient held in a tensor of the caller's own is accumulated into in place:
                 # hand it a copy so the flat buffer can be reused by the next step
                 grads.append(gv.clone() if p.grad is not None else gv)
@@ -1401,8 +1448,9 @@ class FusedAdam(torch.optim.Optimizer):
         o1 = o0 + sum(_round_up(w.numel()) for w in blocks)
         for lo, hi in ((0, o0), (o1, fp.numel)):
             if hi > lo:
-                eng._call("clt_adam_step", fp.flat[lo:hi], fp.grad[lo:hi], fp.exp_avg[lo:hi], fp.exp_avg_sq[lo:hi],
-                          fp.shadow[lo:hi] if fp.shadow is not None else None, hi - lo, *args)
+                at = [t.data_ptr() + 4 * lo for t in (fp.flat, fp.grad, fp.exp_avg, fp.exp_avg_sq)]
+                eng._call("clt_adam_step", *at, fp.shadow.data_ptr() + 2 * lo if fp.shadow is not None else None, hi - lo,
+                          *args)
         for p in group["params"]:
             self.state[p]["step"] = self._step
         eng.decoder_updated = False

@@ -104,6 +104,13 @@ int clt_loss_bwd(const float* recon, const float* aux, const void* batch, int in
                  const float* sd_out, const float* gscale, float aux_scale, void* drecon, void* daux, int bf16,
                  float* db_dec, int B, int L, int D, clt_stream_t stream);
 
+/* Four statistics of n values each, fp16 or bf16 (dtype 1 or 2, as in_dtype), as fp32 one after the other: out [4, n]. */
+int clt_cast_stats(const void* a, const void* b, const void* c, const void* d, int dtype, float* out, int n,
+                   clt_stream_t stream);
+/* Up to four arrays of n0 .. n3 floats are set to zero (NULL with 0: none). */
+int clt_zero4(float* p0, int64_t n0, float* p1, int64_t n1, float* p2, int64_t n2, float* p3, int64_t n3,
+              clt_stream_t stream);
+
 /* clt_loss_bwd for the token rows [b_lo, b_lo + b_cnt) that this rank owns, fused with the all-gather of
  * the result over the feature-shard ranks of one node.  recon_own / aux_own hold the owned rows'
  * summed reconstructions as [b_cnt, L, D]; batch is the whole [B, 2, L, D] batch; the gradient rows are
