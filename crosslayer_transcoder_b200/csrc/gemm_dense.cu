@@ -67,8 +67,10 @@ bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F >
 // Output tiles run `slots` at a time (one to an SM in bf16, two in fp32), so a fair share of the work is
 // total * tiles / slots k-blocks, and the launch lasts as long as its longest chain.  Parts come into question when
 // that chain is over 3/2 of the share: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) whole chains took 170
-// us and parts 200 us.  Parts of half a share keep the last wave short; below 8 blocks a part's output costs more than its
-// products.  Then both forms are estimated (us):
+// us and parts 200 us.  In fp32, parts of half a share keep the last wave short; in bf16 the number of parts is fitted to
+// whole rounds of the chip (12th call of a 12-layer crosslayer decoder, 257 tokens, 9 tiles: 33 parts of half a share were
+// 297 blocks on 148 SMs, a third round for one; 16 parts are one round).  Below 8 blocks a part's output costs
+// more than its products.  Then both forms are estimated (us):
 //   * a bf16 block takes its CTA 0.39 (staging its operands from L2), whatever the tile is filled with;
 //   * fp32: 2.2 in a 128 x 128 tile, two to an SM, 0.62 of the SM's time in a 64 x 64 tile but 0.9 of its own; small
 //     tiles are what whole chains get when the large ones are fewer than the SMs, and what parts often do not get;
@@ -94,10 +96,29 @@ int plan_parts(GemmGeom& g, bool bf16, int sms) {
     longest = n > longest ? n : longest;
   }
   if (longest < 32 || longest * slots * 2 <= total * tiles * 3) return 0;
-  const long long half = up(total * tiles, 2 * slots), part = half < 8 ? 8 : half;
-  g.kb_per_part = (int)part;
-  long long parts = 0;
-  for (int z = 0; z < g.nz; ++z) parts += part_count(g, z, kb_per_seg);
+  const auto count = [&](long long part) {
+    g.kb_per_part = (int)part;
+    long long n = 0;
+    for (int z = 0; z < g.nz; ++z) n += part_count(g, z, kb_per_seg);
+    return n;
+  };
+  long long part = up(total * tiles, 2 * slots), parts;
+  if (bf16) {
+    // the shortest parts that fill 1 .. 4 rounds of the chip without beginning another; the cheapest of them
+    double best = 0;
+    long long best_part = 0;
+    for (int rounds = 1; rounds <= 4; ++rounds) {
+      long long p = up(total * tiles, rounds * slots);
+      if (p < 8) p = 8;
+      for (int i = 0; i < 64 && count(p) * tiles > rounds * slots; ++i) p += 1 + p / 64;
+      const double cost = 0.39 * p * up(count(p) * tiles, slots) + 8.0 * count(p) * g.M * g.N / 5e6;
+      if (best_part == 0 || cost < best) best = cost, best_part = p;
+    }
+    part = best_part;
+  } else if (part < 8) {
+    part = 8;
+  }
+  parts = count(part);
   double whole, split;
   if (bf16) {
     whole = 0.39 * longest;
@@ -181,6 +202,25 @@ int clt_encoder_fwd_store(const void* xn, const void* W_enc, void* z_out, int B,
   epi::StoreZ<bf16_t>::Params p16{(bf16_t*)z_out};
   return run_gemm<epi::StoreZ<float>, epi::StoreZ<bf16_t>, false, true>(g, a, b, p32, p16, bf16, status,
                                                                         (cudaStream_t)stream);
+}
+
+int clt_encoder_layer_fwd(const void* x, int in_dtype, const void* W_enc, const float* b_enc, void* xn, float* out, int B,
+                          int D, int F, int* status, clt_stream_t stream) {
+  CLT_CHECK_ARG(dims_ok(B, 1, D, F), "encoder_layer_fwd: bad dims B=%d D=%d F=%d", B, D, F);
+  CLT_CHECK_ARG(x && W_enc && xn && out && status, "encoder_layer_fwd: null pointer");
+  if (int rc = prep_input(x, in_dtype, nullptr, nullptr, xn, 1, B, 1, D, 1, (cudaStream_t)stream)) return rc;
+  GemmGeom g{kBatched, B, F, D, 1, 1};
+  Operand a{xn, 1, B, D, 1}, b{W_enc, 0, F, D, 1};
+  epi::PreOut<bf16_t>::Params p{out, b_enc};
+  return tc::launch_gemm_tc<epi::PreOut<bf16_t>, false, true>(g, tc_operand(a), tc_operand(b), p, status,
+                                                              device_sm_count(), (cudaStream_t)stream);
+}
+
+int clt_decoder_layer_fwd(const float* x, int64_t ld, const void* W_dec, const float* b_dec, void* feat, float* recon,
+                          float* ws, int64_t ws_floats, int B, int K, int D, int bf16, int* status,
+                          clt_stream_t stream) {
+  if (int rc = clt_import_rows(x, ld, feat, B, K, bf16, stream)) return rc;
+  return clt_decoder_dense_fwd_ws(feat, W_dec, b_dec, recon, ws, ws_floats, B, 1, D, K, 0, bf16, status, stream);
 }
 
 int clt_decoder_dense_fwd(const void* feat, const void* W_dec, const float* b_dec, float* recon, int B, int L, int D,

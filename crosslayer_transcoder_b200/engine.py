@@ -702,6 +702,13 @@ class StepEngine:
         T = torch.bfloat16 if bf16 else torch.float32
         s = stream_ptr()
         xn = torch.empty(1, B, D, dtype=T, device=dev)
+        if bf16 and B * F >= 16384:
+            # the contraction's epilogue writes the result; fewer values than a tile's are launch latency either way
+            out = torch.empty(B, F, dtype=torch.float32, device=dev)
+            self.launches += 1                          # (two kernels in this call)
+            self._call("clt_encoder_layer_fwd", x, DTYPE_CODE[x.dtype], self._operand(enc.W, bf16)[layer],
+                       enc.b.data[layer] if enc.bias else None, xn, out, B, D, F, self.status, s)
+            return out.view(*lead, F)
         self._call("clt_prep_acts", x, DTYPE_CODE[x.dtype], None, None, xn, int(bf16), B, 1, D, s)
         z = torch.empty(1, B, F, dtype=T, device=dev)
         self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16)[layer:layer + 1], z, B, 1, D, F, int(bf16),
@@ -738,13 +745,15 @@ class StepEngine:
         self.prepare(dev, bf16)
         T = torch.bfloat16 if bf16 else torch.float32
         s = stream_ptr()
-        feat = torch.empty(1, B, K, dtype=T, device=dev)
-        self._call("clt_import_rows", x, x.stride(0), feat, B, K, int(bf16), s)
+        feat = torch.empty(B, K, dtype=T, device=dev)
         w_op = self._operand(w, bf16)
-        w_op = w_op.reshape(1, K, D) if dec.crosslayer else w_op[layer:layer + 1]
-        recon = torch.empty(B, 1, D, dtype=torch.float32, device=dev)
-        self._decoder_dense_fwd(feat, w_op, dec.b.data[layer:layer + 1], recon, B, 1, D, K, 0, bf16)
-        return recon.reshape(*lead, D)
+        recon = torch.empty(B, D, dtype=torch.float32, device=dev)
+        n = lib().query("clt_decoder_dense_parts", B, 1, D, K, 0, int(bf16), 0) * B * D
+        ws = torch.empty(n, dtype=torch.float32, device=dev) if n else None      # the call's own, as in _decoder_dense_fwd
+        self.launches += 1                              # (two kernels in this call)
+        self._call("clt_decoder_layer_fwd", x, x.stride(0), w_op if dec.crosslayer else w_op[layer], dec.b.data[layer],
+                   feat, recon, ws, n, B, K, D, int(bf16), self.status, s)
+        return recon.view(*lead, D)
 
     # ------------------------------------------------------------------ backward
     def backward(self, ctx: dict, gscale: torch.Tensor):
