@@ -105,37 +105,87 @@ struct Raw8 {
   }
 };
 
-// same as prep_input_kernel, 8 consecutive d per thread (needs D % 8 == 0).  One warp per (token, layer) row:
-// the 64-bit index arithmetic is done once per row, not once per 16 bytes (which made this copy-like kernel
-// run at half the copy rate).
-template <class TIn, class TOut>
-__global__ void prep_input_vec_kernel(const TIn* __restrict__ batch, const float* __restrict__ mu,
-                                      const float* __restrict__ sd, TOut* __restrict__ xn, int B, int L, int D,
-                                      int halves) {
-  const int dv = D / 8;
-  const int lane = threadIdx.x & 31;
-  const long long rows = (long long)B * L;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarps) {
-    const int l = (int)(r % L);
-    const long long b = r / L;
-    const TIn* src = batch + ((b * halves + 0) * L + l) * (long long)D;
-    TOut* dst = xn + ((long long)l * B + b) * D;
-    const float* ml = mu != nullptr ? mu + (long long)l * D : nullptr;
-    const float* sl = mu != nullptr ? sd + (long long)l * D : nullptr;
-#pragma unroll 4
-    for (int c = lane; c < dv; c += 32) {
-      float x[8];
-      load8<TIn>(src + 8 * c, x);
-      if (ml != nullptr) {
-        float m[8], s[8];
-        load8<float>(ml + 8 * c, m);
-        load8<float>(sl + 8 * c, s);
+// The streaming kernels over the batch (input preparation, loss forward and backward) share one shape: a thread owns 8
+// consecutive (l, d) columns, whose statistics stay in registers, and walks batch rows, kStripRows of them in flight; a
+// CTA of (32, 8) covers 256 columns and a strip of rows.  Every access is 16 bytes a lane.  They are bound by HBM; a warp
+// per (token, layer) row that fetched the statistics again for each (input preparation, loss forward), or 4 columns a
+// thread, one row at a time and 2-byte stores (loss backward) took longer
+// (fp16 batch, bf16 gradients): 4000 x 12 x 768 preparation 51 -> 39 us (5.7 TB/s), forward 55 -> 52, backward 78 -> 62;
+// 8192 x 4 x 2048 78 -> 64, 86 -> 85, 137 -> 102; 136 x 3 x 64 backward 21 -> 8.
+constexpr int kStripRows = 4;
+struct Strip {
+  int c, l, d, b0, b1;  // this thread's first column, its layer and place in it; this thread's first and the CTA's last row
+  __device__ Strip(int B, int D, int rows_per_cta) {
+    c = (blockIdx.x * 32 + threadIdx.x) * 8;
+    l = c / D, d = c - l * D;
+    b0 = blockIdx.y * rows_per_cta + threadIdx.y;
+    b1 = min(B, (int)(blockIdx.y + 1) * rows_per_cta);
+  }
+};
+// rows of a CTA: 8 to a thread; fewer while that leaves SMs without a CTA
+static inline int strip_rows(int B, int LD) {
+  int rows = 64;
+  while (rows > 8 && (long long)((LD / 8 + 31) / 32) * ((B + rows - 1) / rows) < 2 * 148) rows /= 2;
+  return rows;
+}
+static inline dim3 strip_grid(int B, int LD, int rows) { return dim3((LD / 8 + 31) / 32, (B + rows - 1) / rows); }
+static inline bool strip_ok(int B, int L, int D) {
+  return D % 8 == 0 && (long long)L * D < (1ll << 30) && B <= 65535 * 8;
+}
+template <class T>
+struct RawIn {  // 8 elements as they lie in memory
+  static constexpr int kWords = sizeof(T) / 2;
+  uint4 w[kWords];
+  __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) x[q] = (x[q] - m[q]) / s[q];
+    for (int i = 0; i < kWords; ++i) w[i] = __ldcs(reinterpret_cast<const uint4*>(p) + i);
+  }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+    if constexpr (sizeof(T) == 4) {
+      const uint32_t x[8] = {w[0].x, w[0].y, w[0].z, w[0].w, w[kWords - 1].x, w[kWords - 1].y, w[kWords - 1].z,
+                             w[kWords - 1].w};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) o[q] = __uint_as_float(x[q]);
+    } else {
+      const uint32_t x[4] = {w[0].x, w[0].y, w[0].z, w[0].w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        o[2 * q] = to_float<T>(reinterpret_cast<const T*>(&x[q])[0]);
+        o[2 * q + 1] = to_float<T>(reinterpret_cast<const T*>(&x[q])[1]);
       }
-      store8<TOut>(dst + 8 * c, x);
     }
+  }
+};
+
+// same as prep_input_kernel (needs D % 8 == 0)
+template <class TIn, class TOut>
+__global__ void __launch_bounds__(256)
+prep_input_vec_kernel(const TIn* __restrict__ batch, const float* __restrict__ mu, const float* __restrict__ sd,
+                      TOut* __restrict__ xn, int B, int L, int D, int halves, int rows_per_cta) {
+  const Strip t(B, D, rows_per_cta);
+  const int LD = L * D;
+  if (t.c >= LD) return;
+  float m[8], sv[8];
+  if (mu != nullptr) load8<float>(mu + t.c, m), load8<float>(sd + t.c, sv);
+  const TIn* src = batch + t.c;
+  TOut* dst = xn + (long long)t.l * B * D + t.d;
+  const long long ld = (long long)halves * LD;
+  for (int b = t.b0; b < t.b1; b += 8 * kStripRows) {
+    RawIn<TIn> raw[kStripRows];
+#pragma unroll
+    for (int i = 0; i < kStripRows; ++i)
+      if (b + 8 * i < t.b1) raw[i].load(src + (b + 8 * i) * ld);
+#pragma unroll
+    for (int i = 0; i < kStripRows; ++i)
+      if (b + 8 * i < t.b1) {
+        float x[8];
+        raw[i].get(x);
+        if (mu != nullptr) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) x[q] = (x[q] - m[q]) / sv[q];
+        }
+        store8<TOut>(dst + (long long)(b + 8 * i) * D, x);
+      }
   }
 }
 
@@ -143,10 +193,11 @@ template <class TIn, class TOut>
 static int prep_input_t(const void* batch, const float* mu, const float* sd, void* xn, int B, int L, int D,
                         int halves, cudaStream_t s) {
   const int threads = 256;
-  if (D % 8 == 0 && ((uintptr_t)batch | (uintptr_t)xn | (uintptr_t)mu | (uintptr_t)sd) % 16 == 0) {  // (NULL statistics pass)
-    const long long rows = (long long)B * L;                       // one warp per row, 8 warps per CTA
-    const int blocks = (int)min((rows + 7) / 8, (long long)148 * 16);
-    prep_input_vec_kernel<TIn, TOut><<<blocks, threads, 0, s>>>((const TIn*)batch, mu, sd, (TOut*)xn, B, L, D, halves);
+  if (strip_ok(B, L, D) &&
+      ((uintptr_t)batch | (uintptr_t)xn | (uintptr_t)mu | (uintptr_t)sd) % 16 == 0) {  // (NULL statistics pass)
+    const int rows = strip_rows(B, L * D);
+    prep_input_vec_kernel<TIn, TOut><<<strip_grid(B, L * D, rows), dim3(32, 8), 0, s>>>((const TIn*)batch, mu, sd,
+                                                                                         (TOut*)xn, B, L, D, halves, rows);
   } else {
     const long long total = (long long)B * L * D;
     const int blocks = (int)min((total + threads - 1) / threads, (long long)148 * 16);
@@ -219,54 +270,62 @@ __global__ void loss_fwd_kernel(const float* __restrict__ recon, const float* __
   }
 }
 
-// same sums, 8 consecutive (l, d) columns per thread (needs L*D % 8 == 0)
-template <class TIn>
-__global__ void loss_fwd_vec_kernel(const float* __restrict__ recon, const float* __restrict__ aux,
-                                    const TIn* __restrict__ batch, const float* __restrict__ mu,
-                                    const float* __restrict__ sd, float* __restrict__ acc, int B, int L, int D) {
-  const long long LD = (long long)L * D;
-  const long long total = (long long)B * LD / 8;
+// same sums (needs D % 8 == 0)
+template <class TIn, bool kAux>
+__global__ void __launch_bounds__(256)
+loss_fwd_vec_kernel(const float* __restrict__ recon, const float* __restrict__ aux, const TIn* __restrict__ batch,
+                    const float* __restrict__ mu, const float* __restrict__ sd, float* __restrict__ acc, int B, int L,
+                    int D, int rows_per_cta) {
+  const Strip t(B, D, rows_per_cta);
+  const int LD = L * D;
+  constexpr int R = kAux ? 2 : kStripRows;
   float s0 = 0.f, s1 = 0.f;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long e = i * 8;
-    const long long c = e % LD, b = e / LD;
-    float y[8], m[8], sdv[8], r[8];
-    load8<TIn>(batch + (b * 2 + 1) * LD + c, y);
-    load8<float>(mu + c, m);
-    load8<float>(sd + c, sdv);
-    load8<float>(recon + e, r);
-    float diff[8];
+  if (t.c < LD) {
+    float m[8], sv[8];
+    load8<float>(mu + t.c, m);
+    load8<float>(sd + t.c, sv);
+    const TIn* yp = batch + LD + t.c;
+    for (int b = t.b0; b < t.b1; b += 8 * R) {
+      RawIn<TIn> raw[R];
+      RawIn<float> rec[R], ax[kAux ? R : 1];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      diff[q] = r[q] - (y[q] - m[q]) / sdv[q];
-      s0 = fmaf(diff[q], diff[q], s0);
-    }
-    if (aux != nullptr) {
-      float a[8];
-      load8<float>(aux + e, a);
+      for (int i = 0; i < R; ++i)
+        if (b + 8 * i < t.b1) {
+          const long long o = (long long)(b + 8 * i) * LD;
+          raw[i].load(yp + 2 * o);
+          rec[i].load(recon + o + t.c);
+          if constexpr (kAux) ax[i].load(aux + o + t.c);
+        }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float ad = a[q] + diff[q];
-        const float sq = ad * ad;
-        s1 += (sq == sq) ? sq : 0.f;
-      }
+      for (int i = 0; i < R; ++i)
+        if (b + 8 * i < t.b1) {
+          float y[8], r[8], a[8];
+          raw[i].get(y);
+          rec[i].get(r);
+          if constexpr (kAux) ax[i].get(a);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float diff = r[q] - (y[q] - m[q]) / sv[q];
+            s0 = fmaf(diff, diff, s0);
+            if constexpr (kAux) {
+              const float ad = a[q] + diff, sq = ad * ad;
+              s1 += (sq == sq) ? sq : 0.f;
+            }
+          }
+        }
     }
   }
   s0 = warp_sum(s0);
   s1 = warp_sum(s1);
-  __shared__ float sh[2][32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) sh[0][w] = s0, sh[1][w] = s1;
+  __shared__ float sh[2][8];
+  if (threadIdx.x == 0) sh[0][threadIdx.y] = s0, sh[1][threadIdx.y] = s1;
   __syncthreads();
-  if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    s0 = warp_sum(lane < nw ? sh[0][lane] : 0.f);
-    s1 = warp_sum(lane < nw ? sh[1][lane] : 0.f);
-    if (lane == 0) {
-      atomicAdd(acc + 0, s0);
-      if (aux != nullptr) atomicAdd(acc + 1, s1);
-    }
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    s0 = s1 = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s0 += sh[0][w], s1 += sh[1][w];
+    atomicAdd(acc + 0, s0);
+    if (kAux) atomicAdd(acc + 1, s1);
   }
 }
 
@@ -275,14 +334,17 @@ int loss_fwd(const float* recon, const float* aux, const void* batch, int in_dty
   if (B <= 0) return 0;
   const long long total = (long long)B * L * D;
   const int threads = 256;
-  const bool vec = ((long long)L * D) % 8 == 0 &&
+  const bool vec = strip_ok(B, L, D) &&
                    ((uintptr_t)recon | (uintptr_t)aux | (uintptr_t)batch | (uintptr_t)mu | (uintptr_t)sd) % 16 == 0;
-  const long long work = vec ? total / 8 : total;
-  const int blocks = (int)min((work + threads - 1) / threads, (long long)148 * 8);
-#define CLT_LF(TI)                                                                                               \
-  if (vec)                                                                                                       \
-    loss_fwd_vec_kernel<TI><<<blocks, threads, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D);      \
-  else                                                                                                           \
+  const int blocks = (int)min((total + threads - 1) / threads, (long long)148 * 8);
+  const int rows = vec ? strip_rows(B, L * D) : 0;
+  const dim3 grid = vec ? strip_grid(B, L * D, rows) : dim3(blocks), strip(32, 8);
+#define CLT_LF(TI)                                                                                                   \
+  if (vec && aux != nullptr)                                                                                         \
+    loss_fwd_vec_kernel<TI, true><<<grid, strip, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D, rows);  \
+  else if (vec)                                                                                                      \
+    loss_fwd_vec_kernel<TI, false><<<grid, strip, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D, rows); \
+  else                                                                                                               \
     loss_fwd_kernel<TI><<<blocks, threads, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D)
   if (in_dtype == 0) {
     CLT_LF(float);
@@ -402,6 +464,74 @@ __global__ void loss_bwd_vec_kernel(const float* __restrict__ recon, const float
       for (int j = 0; j < (int)blockDim.y; ++j) t += sh[j][threadIdx.x][q];
       if (t != 0.f) atomicAdd(db_dec + c + q, t);
     }
+  }
+}
+
+// same computation (needs D % 8 == 0)
+template <class TIn, class TOut, bool kAux>
+__global__ void __launch_bounds__(256)
+loss_bwd_strip_kernel(const float* __restrict__ recon, const float* __restrict__ aux, const TIn* __restrict__ batch,
+                      const float* __restrict__ mu, const float* __restrict__ sd, const float* __restrict__ gscale,
+                      float aux_scale, TOut* __restrict__ drecon, TOut* __restrict__ daux, float* __restrict__ db_dec,
+                      int B, int L, int D, int rows_per_cta) {
+  const Strip t(B, D, rows_per_cta);
+  const int LD = L * D;
+  constexpr int R = kAux ? 2 : kStripRows;
+  const float gs = (gscale != nullptr ? *gscale : 1.f) / ((float)B * (float)L * (float)D);
+  float cs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (t.c < LD) {
+    float m[8], sv[8];
+    load8<float>(mu + t.c, m);
+    load8<float>(sd + t.c, sv);
+    const TIn* yp = batch + LD + t.c;
+    const long long out0 = (long long)t.l * B * D + t.d;
+    for (int b = t.b0; b < t.b1; b += 8 * R) {
+      RawIn<TIn> raw[R];
+      RawIn<float> rec[R], ax[kAux ? R : 1];
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (b + 8 * i < t.b1) {
+          const long long o = (long long)(b + 8 * i) * LD;
+          raw[i].load(yp + 2 * o);
+          rec[i].load(recon + o + t.c);
+          if constexpr (kAux) ax[i].load(aux + o + t.c);
+        }
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (b + 8 * i < t.b1) {
+          float y[8], r[8], a[8], g[8], ga[8];
+          raw[i].get(y);
+          rec[i].get(r);
+          if constexpr (kAux) ax[i].get(a);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const float diff = r[q] - (y[q] - m[q]) / sv[q];
+            g[q] = 2.f * diff * gs;
+            if constexpr (kAux) {
+              const float ad = a[q] + diff;
+              ga[q] = (ad * ad == ad * ad) ? 2.f * ad * aux_scale * gs : 0.f;
+              g[q] += ga[q];
+              cs[q] += ga[q];
+            }
+            cs[q] += g[q];
+          }
+          const long long o = out0 + (long long)(b + 8 * i) * D;
+          store8<TOut>(drecon + o, g);
+          if constexpr (kAux) store8<TOut>(daux + o, ga);
+        }
+    }
+  }
+  __shared__ float sh[8][32][9];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) sh[threadIdx.y][threadIdx.x][q] = cs[q];
+  __syncthreads();
+  // thread (x, y) adds up column 32 y + x of the CTA's 256
+  const int col = threadIdx.y * 32 + threadIdx.x, c = blockIdx.x * 256 + col;
+  if (c < LD) {
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum += sh[j][col >> 3][col & 7];
+    if (sum != 0.f) atomicAdd(db_dec + c, sum);
   }
 }
 
@@ -585,8 +715,19 @@ int loss_bwd(const float* recon, const float* aux, const void* batch, int in_dty
   const int rows_per_cta = 256;
   const bool vec = D % 4 == 0 && ((uintptr_t)recon | (uintptr_t)aux | (uintptr_t)mu | (uintptr_t)sd) % 16 == 0;
   dim3 grid(vec ? (LD / 4 + 31) / 32 : (LD + 31) / 32, (B + rows_per_cta - 1) / rows_per_cta), block(32, 8);
+  const bool strips = vec && strip_ok(B, L, D) && ((uintptr_t)batch | (uintptr_t)drecon | (uintptr_t)daux) % 16 == 0;
+  // fp32 steps add the bias gradient up in the order in which the kernels below do (256 rows to a CTA): what follows
+  // from its last bits reaches thresholds
+  const int rows = !strips ? 0 : out_bf16 ? strip_rows(B, LD) : 256;
+  const dim3 sgrid = strips ? strip_grid(B, LD, rows) : dim3(1);
 #define CLT_LB(TI, TO)                                                                                            \
-  if (vec)                                                                                                        \
+  if (strips && aux != nullptr)                                                                                   \
+    loss_bwd_strip_kernel<TI, TO, true><<<sgrid, block, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, gscale,     \
+        aux_scale, (TO*)drecon, (TO*)daux, db_dec, B, L, D, rows);                                                \
+  else if (strips)                                                                                                \
+    loss_bwd_strip_kernel<TI, TO, false><<<sgrid, block, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, gscale,    \
+        aux_scale, (TO*)drecon, (TO*)daux, db_dec, B, L, D, rows);                                                \
+  else if (vec)                                                                                                      \
     loss_bwd_vec_kernel<TI, TO><<<grid, block, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, gscale, aux_scale,   \
                                                        (TO*)drecon, (TO*)daux, db_dec, B, L, D, rows_per_cta);    \
   else                                                                                                            \

@@ -1,0 +1,47 @@
+"""Input preparation, loss forward and loss backward against float64, at the ends of their column blocks and row strips,
+for rows that are and are not multiples of 8 columns."""
+import pytest
+import torch
+
+from crosslayer_transcoder_b200._lib import DTYPE_CODE, lib, stream_ptr
+
+pytestmark = pytest.mark.gpu
+
+
+# 256 columns to a CTA, strips of 8 to 64 rows (256 in fp32), 2 or 4 rows in flight per thread
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,L,D", [(1, 1, 8), (9, 3, 88), (31, 2, 128), (65, 5, 72), (300, 2, 264), (2049, 1, 16),
+                                   (33, 3, 20)])
+def test_against_float64(B, L, D, dtype, out):
+    g = torch.Generator(device="cuda:0").manual_seed(B + D)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda:0")
+    batch, mu, sd = r(B, 2, L, D).to(dtype), 0.3 * r(L, D), 0.5 + r(L, D).abs()
+    recon, aux, s, code, bf16 = r(B, L, D), 0.1 * r(B, L, D), stream_ptr(), DTYPE_CODE[dtype], int(out == torch.bfloat16)
+    xn = torch.empty(L, B, D, dtype=out, device="cuda:0")
+    lib().call("clt_prep_input", batch, code, mu, sd, xn, bf16, B, L, D, s)
+    # the subtraction and the division of the same fp32 values, rounded once more to the output's type
+    assert torch.equal(xn, ((batch[:, 0].float() - mu) / sd).to(out).transpose(0, 1))
+    y = (batch[:, 1].double() - mu.double()) / sd.double()
+    diff = recon.double() - y
+    n, scale = float(B * L * D), 1 / 32
+    for a in (None, aux):
+        acc = torch.zeros(2, device="cuda:0")
+        lib().call("clt_loss_fwd", recon, a, batch, code, mu, sd, acc, B, L, D, s)
+        want = torch.stack([(diff ** 2).sum(), ((aux.double() + diff) ** 2).sum() if a is not None else diff.new_zeros(())])
+        assert torch.allclose(acc.double(), want, rtol=1e-5)
+        dr, da = torch.empty_like(xn), torch.empty_like(xn)
+        db, gs = torch.zeros(L, D, device="cuda:0"), torch.full((1,), 3.0, device="cuda:0")
+        lib().call("clt_loss_bwd", recon, a, batch, code, mu, sd, gs, scale if a is not None else 0.0, dr,
+                   da if a is not None else None, bf16, db, B, L, D, s)
+        ga = 2 * (aux.double() + diff) * scale * 3.0 / n if a is not None else torch.zeros_like(diff)
+        gr = 2 * diff * 3.0 / n + ga
+        # a few fp32 roundings of the terms (y, diff and the products), then the output's: half a bf16 step is 2^-8 of a
+        # value, and no gradient is larger than its terms' magnitudes with the auxiliary share on top
+        tol = (2.0 ** -8 if bf16 else 0.0) + 2.0 ** -20
+        mag = recon.double().abs() + batch[:, 1].double().abs() / sd + mu.abs() / sd + aux.abs()
+        mag = 2 * (1 + scale) * mag * 3.0 / n
+        assert bool(((dr.transpose(0, 1).double() - gr).abs() <= tol * mag).all())
+        if a is not None:
+            assert bool(((da.transpose(0, 1).double() - ga).abs() <= tol * mag).all())
+        assert bool(((db.double() - (gr + ga).sum(0)).abs() <= 2.0 ** -20 * 2 * mag.sum(0)).all())
