@@ -94,6 +94,24 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// Sum of `v` (uniform over a warp) of the warps before this one, and of all; 1024 threads.
+__device__ __forceinline__ int block1024_offset(int v, int& all) {
+  __shared__ int warp_values[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) warp_values[w] = v;
+  __syncthreads();
+  int x = warp_values[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  all = __shfl_sync(0xffffffffu, x, 31);
+  const int before = __shfl_sync(0xffffffffu, x, w) - v;
+  __syncthreads();  // the array may be written again
+  return before;
+}
+
 // Column sums over the 32 rows held by one warp.  Each lane holds 32 values
 // (one row, 32 consecutive columns); on return lane j holds the sum over all
 // lanes of column j.  Recursive halving: 31 shuffles for 32 columns.

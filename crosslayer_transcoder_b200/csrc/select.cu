@@ -676,35 +676,36 @@ select_topk_stream_kernel(const T* __restrict__ z, const float* __restrict__ b_e
 
 // ---------------------------------------------------------------------------------------
 // Dead-feature list per layer: dead_list[l, 0..n_dead[l]) = ascending indices with dead != 0.
-// One CTA per layer.
+// One CTA of 1024 threads per layer, a warp 256 consecutive flags per round, as in the counting sort's scan; one flag per
+// thread and round and a serial sum over the warps took 53 us where this takes 12 (12 x 32768; 12 x 20000: 35 -> 10).
 // ---------------------------------------------------------------------------------------
-__global__ void dead_compact_kernel(const unsigned char* __restrict__ dead, int* __restrict__ dead_list,
-                                    int* __restrict__ n_dead, int F) {
+__global__ void __launch_bounds__(1024)
+dead_compact_kernel(const unsigned char* __restrict__ dead, int* __restrict__ dead_list, int* __restrict__ n_dead, int F) {
+  constexpr int kRows = 8;
   const int l = blockIdx.x;
-  __shared__ int base;
-  __shared__ int wsum[32];
-  if (threadIdx.x == 0) base = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int f0 = 0; f0 < F; f0 += blockDim.x) {
-    const int f = f0 + threadIdx.x;
-    const int flag = (f < F && dead[(size_t)l * F + f]) ? 1 : 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, flag);
-    const int before = __popc(bal & ((1u << lane) - 1u));
-    if (lane == 0) wsum[w] = __popc(bal);
-    __syncthreads();
-    int woff = 0;
-    for (int j = 0; j < w; ++j) woff += wsum[j];
-    if (flag) dead_list[(size_t)l * F + base + woff + before] = f;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int j = 0; j < nw; ++j) tot += wsum[j];
-      base += tot;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned char* dl = dead + (size_t)l * F;
+  int* out = dead_list + (size_t)l * F;
+  int count = 0;
+  for (int f0 = 0; f0 < F; f0 += 1024 * kRows) {
+    const int base = f0 + w * 32 * kRows + lane;
+    bool flag[kRows];
+    unsigned bal[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) flag[j] = base + 32 * j < F && dl[base + 32 * j] != 0;
+    int total = 0;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) bal[j] = __ballot_sync(0xffffffffu, flag[j]), total += __popc(bal[j]);
+    int all;
+    int at = count + block1024_offset(total, all);
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      if (flag[j]) out[at + __popc(bal[j] & ((1u << lane) - 1u))] = base + 32 * j;
+      at += __popc(bal[j]);
     }
-    __syncthreads();
+    count += all;
   }
-  if (threadIdx.x == 0) n_dead[l] = base;
+  if (threadIdx.x == 0) n_dead[l] = count;
 }
 
 // ---------------------------------------------------------------------------------------

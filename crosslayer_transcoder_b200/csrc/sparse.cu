@@ -386,34 +386,40 @@ __global__ void csc_count_kernel(const int* __restrict__ idx, const float* __res
   }
 }
 
-// exclusive scan of count[l, 0..F) in place -> col_ptr[l, 0..F]; cursor[l, f] = col_ptr[l, f]
-__global__ void csc_scan_kernel(int* __restrict__ col_ptr, int* __restrict__ cursor, int F) {
+// exclusive scan of count[l, 0..F) in place -> col_ptr[l, 0..F]; cursor[l, f] = col_ptr[l, f].  One CTA of 1024 threads
+// per layer, a warp 256 consecutive counts per round (8 coalesced loads in flight).  Latency-bound, so few rounds: one
+// count per thread and round and a serial sum over the warps: the whole sort 77 -> 56 us at 12 x 32768, 44 -> 33 at 12 x 20000.
+__global__ void __launch_bounds__(1024) csc_scan_kernel(int* __restrict__ col_ptr, int* __restrict__ cursor, int F) {
+  constexpr int kRows = 8;
   const int l = blockIdx.x;
   int* cp = col_ptr + (size_t)l * (F + 1);
   int* cur = cursor + (size_t)l * F;
-  __shared__ int wsum[32];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int f0 = 0; f0 < F; f0 += blockDim.x) {
-    const int f = f0 + threadIdx.x;
-    const int c = f < F ? cp[f] : 0;
-    int x = c;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int carry = 0;
+  for (int f0 = 0; f0 < F; f0 += 1024 * kRows) {
+    const int base = f0 + w * 32 * kRows + lane;
+    int c[kRows], x[kRows];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+    for (int j = 0; j < kRows; ++j) c[j] = base + 32 * j < F ? cp[base + 32 * j] : 0;
+    int total = 0;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      x[j] = c[j];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x[j], o);
+        if (lane >= o) x[j] += y;
+      }
+      const int row = __shfl_sync(0xffffffffu, x[j], 31);
+      x[j] += total - c[j];
+      total += row;
     }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    int woff = 0;
-    for (int j = 0; j < w; ++j) woff += wsum[j];
-    const int excl = carry + woff + x - c;
-    __syncthreads();
-    if (f < F) cp[f] = excl, cur[f] = excl;
-    if (threadIdx.x == blockDim.x - 1) carry = excl + c;
-    __syncthreads();
+    int all;
+    const int before = carry + block1024_offset(total, all);
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+      if (base + 32 * j < F) cp[base + 32 * j] = cur[base + 32 * j] = before + x[j];
+    carry += all;
   }
   if (threadIdx.x == 0) cp[F] = carry;
 }
