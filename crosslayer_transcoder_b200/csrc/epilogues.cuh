@@ -203,13 +203,42 @@ __device__ __forceinline__ void store_rows32<float>(unsigned char* stage, float*
   }
 }
 
-// Store a warp's sub-tile: coalesced through `stage` when the 32 columns are all inside the matrix
-// and rows are 16-byte aligned, else lane by lane with guards.  `row0` is the warp's first row.
-template <class T>
+// The same for fp32 rows that are not 16-byte aligned, or that end inside the sub-tile: 2 rows x 16 columns to an
+// instruction, so that it touches 4 to 6 sectors where a row per lane touches 32 (6 x 777 tokens x 320 x 2001 fp32:
+// encoder 230 -> 190 us, with the (Jump)ReLU 302 -> 230, feature gradient 267 -> 238).
+__device__ __forceinline__ void store_rows32_scalar(unsigned char* stage, float* base, size_t ld, int rows_valid,
+                                                    int cols_valid, const float (&v)[32]) {
+  const int lane = threadIdx.x & 31, c = lane & 15;
+  float4* mine = reinterpret_cast<float4*>(stage + lane * kStageRow);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      mine[i] = make_float4(v[16 * h + 4 * i], v[16 * h + 4 * i + 1], v[16 * h + 4 * i + 2], v[16 * h + 4 * i + 3]);
+    __syncwarp();
+    if (16 * h + c < cols_valid) {
+#pragma unroll
+      for (int it = 0; it < 16; ++it) {
+        const int r = it * 2 + (lane >> 4);
+        const float t = *reinterpret_cast<const float*>(stage + r * kStageRow + c * 4);
+        if (r < rows_valid) base[(size_t)r * ld + 16 * h + c] = t;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// Store a warp's sub-tile through `stage`, in 16-byte pieces when the 32 columns are all inside the matrix and rows are
+// 16-byte aligned; others lane by lane with guards.  kOdd: fp32 rows may end anywhere (feature counts do; widths hardly
+// ever, and for them the second way through `stage` cost the CUDA-core kernel 3 % in spilled registers).  `row0` is the
+// warp's first row.
+template <class T, bool kOdd = false>
 __device__ __forceinline__ void store_tile(unsigned char* stage, T* mat, size_t ld, int row0, int row, bool row_ok,
                                            int M, int n0, int N, bool aligned, const float (&v)[32]) {
   if (aligned && n0 + 32 <= N) {
     store_rows32<T>(stage, mat + (size_t)row0 * ld + n0, ld, M - row0, v);
+  } else if constexpr (kOdd && sizeof(T) == 4) {
+    store_rows32_scalar(stage, mat + (size_t)row0 * ld + n0, ld, M - row0, N - n0, v);
   } else if (row_ok) {
     store32<T>(mat + (size_t)row * ld + n0, N - n0, false, v);
   }
@@ -274,6 +303,30 @@ __device__ __forceinline__ void load_rows32<float>(unsigned char* stage, const f
   }
 }
 
+// The mirror image of store_rows32_scalar; what lies outside reads as 0.
+__device__ __forceinline__ void load_rows32_scalar(unsigned char* stage, const float* base, size_t ld, int rows_valid,
+                                                   int cols_valid, float (&o)[32]) {
+  const int lane = threadIdx.x & 31, c = lane & 15;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int it = 0; it < 16; ++it) {
+      const int r = it * 2 + (lane >> 4);
+      float t = 0.f;
+      if (r < rows_valid && 16 * h + c < cols_valid) t = base[(size_t)r * ld + 16 * h + c];
+      *reinterpret_cast<float*>(stage + r * kStageRow + c * 4) = t;
+    }
+    __syncwarp();
+    const float4* mine = reinterpret_cast<const float4*>(stage + lane * kStageRow);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 t = mine[i];
+      o[16 * h + 4 * i] = t.x, o[16 * h + 4 * i + 1] = t.y, o[16 * h + 4 * i + 2] = t.z, o[16 * h + 4 * i + 3] = t.w;
+    }
+    __syncwarp();
+  }
+}
+
 // lane j adds its column total to dst[n0 + j]
 __device__ __forceinline__ void col_atomic_add(float* dst, int n0, int N, float colsum) {
   const int lane = threadIdx.x & 31;
@@ -298,7 +351,7 @@ struct StoreZ {
   __device__ static void apply(const Params& p, State&, int z, int row, bool row_ok, int n0, int M, int N,
                                float (&v)[32], const float*, unsigned char* stage) {
     const int row0 = row - (threadIdx.x & 31);
-    store_tile<T>(stage, p.out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N,
+    store_tile<T, true>(stage, p.out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N,
                   N % (16 / (int)sizeof(T)) == 0, v);
   }
   __device__ static void finish(const Params&, State&) {}
@@ -590,8 +643,8 @@ struct EncJumpReLU {
     }
     const int row0 = row - (threadIdx.x & 31);
     const bool al = N % (16 / (int)sizeof(T)) == 0;
-    store_tile<T>(stage, p.z_out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N, al, v);
-    store_tile<T>(stage, p.feat_out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N, al, feat);
+    store_tile<T, true>(stage, p.z_out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N, al, v);
+    store_tile<T, true>(stage, p.feat_out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N, al, feat);
   }
   __device__ static void finish(const Params& p, State& st) {
     const float a = warp_sum(st.s_pre), b = warp_sum(st.s_sp);
@@ -652,6 +705,8 @@ struct DFeatJumpReLU {
     float zv[32];
     if (al && n0 + 32 <= N) {
       load_rows32<T>(stage, p.z_in + ((size_t)z * M + row0) * N + n0, (size_t)N, M - row0, zv);
+    } else if constexpr (sizeof(T) == 4) {
+      load_rows32_scalar(stage, p.z_in + ((size_t)z * M + row0) * N + n0, (size_t)N, M - row0, N - n0, zv);
     } else {
       const size_t off = ((size_t)z * M + (row_ok ? row : 0)) * N + n0;
       load32<T>(p.z_in + off, row_ok ? N - n0 : 0, false, zv);
@@ -665,7 +720,7 @@ struct DFeatJumpReLU {
       if (edge) body<CS, false, true>(p, row_ok, n0, N, v, zv, dth, dnr, colp);
       else body<CS, false, false>(p, row_ok, n0, N, v, zv, dth, dnr, colp);
     }
-    store_tile<T>(stage, p.dpre_out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N, al, v);
+    store_tile<T, true>(stage, p.dpre_out + (size_t)z * M * N, (size_t)N, row0, row, row_ok, M, n0, N, al, v);
     col_atomic_add(p.dbenc + (size_t)z * N, n0, N, warp_colsum32(v));
     if (p.dtheta != nullptr) col_atomic_add(p.dtheta + (size_t)z * N, n0, N, warp_colsum32(dth));
     if (sp && p.dnorm != nullptr) col_atomic_add(p.dnorm + (size_t)z * N, n0, N, warp_colsum32(dnr));
