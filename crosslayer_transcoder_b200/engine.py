@@ -139,6 +139,7 @@ class StepEngine:
         self.profile: Optional[dict] = None
         self._library = None
         self._sum_views: Dict[str, tuple] = {}    # see _sums
+        self._last_ctx: Optional[dict] = None     # of the step whose buffers the workspace holds
         # the device status word is copied to pinned host memory after every backward and looked at,
         # without waiting, when the next steps begin
         self.optimizer = None                     # the FusedAdam of configure_optimizers (for fuse_optimizer)
@@ -339,7 +340,7 @@ class StepEngine:
         normalised reconstruction and L0 (overall and per layer).  Two kernels reduce buffers the step
         already holds (``clt_recon_stats``, ``clt_count_active``); nothing is copied to the host.  On feature
         shards every rank gets the figures of the whole model."""
-        c = getattr(self, "_last_ctx", None)
+        c = self._last_ctx
         if c is None:
             raise CltError("training_metrics() needs a training step to have run")
         B, L, D, F = c["B"], c["L"], c["D"], c["F"]
@@ -465,6 +466,11 @@ class StepEngine:
         """(loss scalar, its four summands): tensors of this step's own."""
         return torch.empty((), dtype=torch.float32, device=dev), torch.empty(4, dtype=torch.float32, device=dev)
 
+    def _begin_step(self):
+        """The workspace, for a step's forward half to write: from here on no earlier step can go backward."""
+        self._last_ctx = None
+        return self.ws
+
     def _sums(self, name: str, n: int, parts: int, shape, dev):
         """Reconstruction buffer ``name`` of ``parts`` x ``n`` floats with a tail of 8 loss sums, in one allocation that
         feature shards reduce together: (whole, [the parts as ``shape``], tail, tail[0:2], tail[2:4])."""
@@ -512,7 +518,7 @@ class StepEngine:
         s = stream_ptr()
         crosslayer = 1 if dec.crosslayer else 0
         mu_i, sd_i, mu_o, sd_o = self._stats()
-        ws = self.ws
+        ws = self._begin_step()
         xn = ws.get("xn", (L, B, D), T, dev)
         z = ws.get("z", (L, B, F), T, dev)
         feat = ws.get("feat", (L, B, F), T, dev)
@@ -757,6 +763,11 @@ class StepEngine:
 
     # ------------------------------------------------------------------ backward
     def backward(self, ctx: dict, gscale: torch.Tensor):
+        # The kernels below read what the forward half left in the workspace; a later step has written there since, and
+        # has made buffers anew where its batch size differs.
+        if ctx is not self._last_ctx:
+            raise CltError("backward() of a step whose buffers a later training step has overwritten: run the backward "
+                           "of a step before the next step's forward")
         if ctx["kind"] in ("jumprelu", "relu"):
             self._backward_dense(ctx, gscale)
         elif ctx["kind"] in ("topk", "batchtopk"):
@@ -789,7 +800,7 @@ class StepEngine:
         s = stream_ptr()
         ws = self.ws
         xn, z, feat = ws.buf["xn"], ws.buf["z"], ws.buf["feat"]
-        _, (recon,), *_ = self._sums("recon", B * L * D, 1, (B, L, D), dev)
+        _, (recon,), *_ = self._sum_views["recon"]
         drecon = ws.get("drecon", (L, B, D), T, dev)
         dpre = ws.get("dpre", (L, B, F), T, dev)
         _, _, mu_o, sd_o = c["stats"]
@@ -854,7 +865,7 @@ class StepEngine:
         s = stream_ptr()
         crosslayer = 1 if dec.crosslayer else 0
         mu_i, sd_i, mu_o, sd_o = self._stats()
-        ws = self.ws
+        ws = self._begin_step()
         xn = ws.get("xn", (L, B, D), T, dev)
         z = ws.get("z", (L, B, F), T, dev)
         # [reconstruction | auxiliary reconstruction | 8-float tail of loss sums]: the first two are
@@ -1037,7 +1048,7 @@ class StepEngine:
         s = stream_ptr()
         crosslayer = 1 if dec.crosslayer else 0
         mu_i, sd_i, mu_o, sd_o = self._stats()
-        ws = self.ws
+        ws = self._begin_step()
         world, group = getattr(mod, "tp_world", 1), getattr(mod, "tp_group", None)
         rank = getattr(mod, "tp_rank", 0)
         bias = dec.b.data if rank == 0 else None
@@ -1175,8 +1186,7 @@ class StepEngine:
         s = stream_ptr()
         ws = self.ws
         xn = ws.buf["xn"]
-        n_rec = B * L * D
-        _, (recon, aux_recon), *_ = self._sums("recon2", n_rec, 2, (B, L, D), dev)
+        _, (recon, aux_recon), *_ = self._sum_views["recon2"]
         aux = c["aux"]
         drecon = ws.get("drecon", (L, B, D), T, dev)
         daux = ws.get("daux", (L, B, D), T, dev) if aux is not None else None

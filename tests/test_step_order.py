@@ -1,0 +1,93 @@
+"""The backward half of a step reads the buffers that its forward half wrote: it is refused, before anything is launched,
+once another step's forward has been given them."""
+import pytest
+import torch
+
+from crosslayer_transcoder_b200 import engine, synthetic
+from crosslayer_transcoder_b200._lib import CltError
+
+from helpers import build_module, spec_inputs
+
+KINDS = ["jumprelu", "topk", "batchtopk", "perlayer_batchtopk"]
+
+
+class _OnDevice(torch.Tensor):
+    """A CPU tensor that says it is on the GPU."""
+    is_cuda = True
+
+
+class _Calls:
+    """In the place of the library: records what would be launched."""
+
+    def __init__(self):
+        self.names = []
+
+    def check_device(self):
+        pass
+
+    def call(self, name, *args):
+        self.names.append(name)
+
+    def query(self, name, *args):
+        return 0
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    rec = _Calls()
+    monkeypatch.setattr(engine, "lib", lambda: rec)
+    monkeypatch.setattr(engine, "stream_ptr", lambda: 0)
+    return rec
+
+
+def _module(kind, dev):
+    spec = synthetic.WorkloadSpec("order", 3, 64, 128, 40, kind, True, False, rank_u=8, n_outlier=1, k=4, k_aux=0)
+    batch, w, la = spec_inputs(spec)
+    mod = build_module(spec, w, dev, last_active=la)
+    batch = batch.to(dev)
+    mod.model.initialize_standardizers(batch)
+    return mod, batch
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("first,second", [(40, 31), (31, 40), (40, 40)])
+def test_earlier_step_is_refused_before_any_launch(kind, first, second, calls):
+    mod, batch = _module(kind, "cpu")
+    batch = batch.as_subclass(_OnDevice)
+    l1 = mod.training_step(batch[:first], 1)
+    mod.training_step(batch[:second], 2)
+    n = len(calls.names)
+    with pytest.raises(CltError, match="overwritten"):
+        l1.backward()
+    assert len(calls.names) == n
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_step_that_failed_half_way_leaves_none_to_go_backward(kind, calls):
+    """The buffers belong to the step that began to write them, whether it came to its end or not."""
+    mod, batch = _module(kind, "cpu")
+    batch = batch.as_subclass(_OnDevice)
+    l1 = mod.training_step(batch, 1)
+    calls.call = lambda name, *args: (_ for _ in ()).throw(CltError("launch failed"))
+    with pytest.raises(CltError, match="launch failed"):
+        mod.training_step(batch[:31], 2)
+    with pytest.raises(CltError, match="overwritten"):
+        l1.backward()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_last_step_still_goes_backward(kind):
+    mod, batch = _module(kind, "cuda:0")
+    mod.training_step(batch[:31], 1).backward()
+    want = [p.grad.clone() for p in mod.parameters()]
+    mod.zero_grad()
+    l1 = mod.training_step(batch, 1)
+    l2 = mod.training_step(batch[:31], 1)
+    with pytest.raises(CltError, match="overwritten"):
+        l1.backward()
+    l2.backward()
+    mod._engine.check_status("step order")
+    for p, w in zip(mod.parameters(), want):
+        # sums by atomics come in another order
+        assert torch.allclose(p.grad, w, rtol=1e-4, atol=1e-6 * float(w.abs().max()) + 1e-12)
