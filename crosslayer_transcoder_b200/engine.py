@@ -60,7 +60,7 @@ class FlatParams:
         self._operands: Dict[int, torch.Tensor] = {}
         # views of this object's own buffers, made once: a slice and a view cost 5 us, a step used two dozen
         self._grads: Dict[int, torch.Tensor] = {}
-        self._decoder: Dict[bool, tuple] = {}
+        self._decoder: Dict[bool, tuple] = {}       # (the blocks, their views): see _dec_flat
         self._strided = [(p.shape, p.data.stride(), self.offsets[id(p)]) for p in self.params]
         if want_bf16:
             self.ensure_shadow()
@@ -261,11 +261,14 @@ class StepEngine:
     def _dec_flat(self, bf16: bool):
         """(operand buffer [P,F,D], fp32 master [P,F,D], gradient [P,F,D]) of the decoder blocks;
         they are adjacent in the flat buffer in block order."""
-        cached = self.flat._decoder.get(bf16)
-        if cached is not None:
-            return cached
         dec = self.module.model.decoder
         blocks = dec.blocks()
+        of, views = self.flat._decoder.get(bf16, ((), None))
+        if len(of) == len(blocks) and all(a is b for a, b in zip(of, blocks)):
+            return views
+        if any(id(w) not in self.flat.offsets for w in blocks):
+            raise CltError("a decoder block is not the parameter that was packed into the flat buffer (replaced by an "
+                           "assignment or by load_state_dict(assign=True)?): copy into the parameters instead")
         F, D = dec.d_features, dec.d_acts
         o0 = self.flat.offsets[id(blocks[0])]
         n = 0
@@ -279,7 +282,7 @@ class StepEngine:
         sl = slice(o0, o0 + n)
         op = (self.flat.shadow if bf16 else self.flat.flat)[sl].view(P, F, D)
         views = op, self.flat.flat[sl].view(P, F, D), self.flat.grad[sl].view(P, F, D)
-        self.flat._decoder[bf16] = views
+        self.flat._decoder[bf16] = tuple(blocks), views
         return views
 
     def _stats(self):

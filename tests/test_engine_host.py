@@ -1,5 +1,4 @@
-"""The backward half of a step reads the buffers that its forward half wrote: it is refused, before anything is launched,
-once another step's forward has been given them."""
+"""What the engine checks on the host before it launches anything; on the CPU with the library replaced by a recorder."""
 import pytest
 import torch
 
@@ -52,6 +51,7 @@ def _module(kind, dev):
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("first,second", [(40, 31), (31, 40), (40, 40)])
 def test_earlier_step_is_refused_before_any_launch(kind, first, second, calls):
+    """The backward half of a step reads the buffers that its forward half wrote; another step's forward now has them."""
     mod, batch = _module(kind, "cpu")
     batch = batch.as_subclass(_OnDevice)
     l1 = mod.training_step(batch[:first], 1)
@@ -73,6 +73,22 @@ def test_step_that_failed_half_way_leaves_none_to_go_backward(kind, calls):
         mod.training_step(batch[:31], 2)
     with pytest.raises(CltError, match="overwritten"):
         l1.backward()
+
+
+@pytest.mark.parametrize("kind", ["jumprelu", "topk"])
+@pytest.mark.parametrize("replace", ["one", "all"])
+def test_replaced_decoder_blocks_are_not_answered_with_the_old_ones(kind, replace, calls):
+    mod, batch = _module(kind, "cpu")
+    acts = batch[:, 0].as_subclass(_OnDevice)
+    dec = mod.model.decoder
+    with torch.no_grad():
+        mod(acts)
+        if replace == "all":
+            dec.load_state_dict({k: v + 1 for k, v in dec.state_dict().items()}, assign=True)
+        else:
+            dec.W_1 = torch.nn.Parameter(dec.W_1.detach() + 1)
+        with pytest.raises(CltError, match="decoder block"):
+            mod(acts)
 
 
 @pytest.mark.gpu
