@@ -137,7 +137,6 @@ class StepEngine:
         self.launches = 0                         # kernels launched by this engine (for reporting)
         self.last_terms: Optional[torch.Tensor] = None
         self.profile: Optional[dict] = None
-        self._library = None
         self._sum_views: Dict[str, tuple] = {}    # see _sums
         self._last_ctx: Optional[dict] = None     # of the step whose buffers the workspace holds
         # the device status word is copied to pinned host memory after every backward and looked at,
@@ -159,7 +158,7 @@ class StepEngine:
         dict, CUDA events around the call collect per-entry-point device time (``tag`` keeps apart two uses
         of one entry point with different shapes)."""
         if self.profile is None:
-            (self._library or self._bind()).call(name, *args)
+            lib().call(name, *args)
         else:
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
@@ -167,10 +166,6 @@ class StepEngine:
             e1.record()
             self.profile.setdefault(name + tag, []).append((e0, e1))
         self.launches += 1
-
-    def _bind(self):
-        self._library = lib()
-        return self._library
 
     def profile_summary(self) -> Dict[str, dict]:
         """{entry point: {"launches", "ms_total", "ms_avg"}} from the collected events (synchronises)."""

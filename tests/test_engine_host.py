@@ -1,8 +1,11 @@
 """What the engine checks on the host before it launches anything; on the CPU with the library replaced by a recorder."""
+import copy
+import pickle
+
 import pytest
 import torch
 
-from crosslayer_transcoder_b200 import engine, synthetic
+from crosslayer_transcoder_b200 import _lib, engine, synthetic
 from crosslayer_transcoder_b200._lib import CltError
 
 from helpers import build_module, spec_inputs
@@ -89,6 +92,20 @@ def test_replaced_decoder_blocks_are_not_answered_with_the_old_ones(kind, replac
             dec.W_1 = torch.nn.Parameter(dec.W_1.detach() + 1)
         with pytest.raises(CltError, match="decoder block"):
             mod(acts)
+
+
+@pytest.mark.parametrize("how", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))], ids=["deepcopy", "pickle"])
+def test_module_that_has_run_can_be_copied(how, monkeypatch):
+    """Weight averaging copies a module, spawned workers pickle it: the engine holds nothing of the loaded library."""
+    monkeypatch.setattr(_lib._Lib, "check_device", lambda self: None)
+    monkeypatch.setattr(_lib._Lib, "call", lambda self, name, *args: None)
+    monkeypatch.setattr(engine, "stream_ptr", lambda: 0)
+    mod, batch = _module("topk", "cpu")
+    with torch.no_grad():
+        mod(batch[:, 0].as_subclass(_OnDevice))
+    other = how(mod)
+    for a, b in zip(mod.parameters(), other.parameters()):
+        assert torch.equal(a, b) and a.data_ptr() != b.data_ptr()
 
 
 @pytest.mark.gpu
