@@ -705,20 +705,21 @@ class StepEngine:
         self.prepare(dev, bf16)
         T = torch.bfloat16 if bf16 else torch.float32
         s = stream_ptr()
+        at = slice(layer, layer + 1)        # empty, which the library refuses, where there is no such layer
         xn = torch.empty(1, B, D, dtype=T, device=dev)
         if bf16 and B * F >= 16384:
             # the contraction's epilogue writes the result; fewer values than a tile's are launch latency either way
             out = torch.empty(B, F, dtype=torch.float32, device=dev)
             self.launches += 1                          # (two kernels in this call)
-            self._call("clt_encoder_layer_fwd", x, DTYPE_CODE[x.dtype], self._operand(enc.W, bf16)[layer],
-                       enc.b.data[layer] if enc.bias else None, xn, out, B, D, F, self.status, s)
+            self._call("clt_encoder_layer_fwd", x, DTYPE_CODE[x.dtype], self._operand(enc.W, bf16)[at],
+                       enc.b.data[at] if enc.bias else None, xn, out, B, D, F, self.status, s)
             return out.view(*lead, F)
         self._call("clt_prep_acts", x, DTYPE_CODE[x.dtype], None, None, xn, int(bf16), B, 1, D, s)
         z = torch.empty(1, B, F, dtype=T, device=dev)
-        self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16)[layer:layer + 1], z, B, 1, D, F, int(bf16),
+        self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16)[at], z, B, 1, D, F, int(bf16),
                    self.status, s)
         out = torch.empty(B, 1, F, dtype=torch.float32, device=dev)
-        self._call("clt_export_blf", z, enc.b.data[layer:layer + 1] if enc.bias else None, out, B, 1, F, int(bf16), s)
+        self._call("clt_export_blf", z, enc.b.data[at] if enc.bias else None, out, B, 1, F, int(bf16), s)
         return out.reshape(*lead, F)
 
     def decode_layer(self, features: torch.Tensor, layer: int) -> torch.Tensor:
@@ -749,13 +750,14 @@ class StepEngine:
         self.prepare(dev, bf16)
         T = torch.bfloat16 if bf16 else torch.float32
         s = stream_ptr()
+        at = slice(layer, layer + 1)        # as in encode_layer
         feat = torch.empty(B, K, dtype=T, device=dev)
         w_op = self._operand(w, bf16)
         recon = torch.empty(B, D, dtype=torch.float32, device=dev)
         n = lib().query("clt_decoder_dense_parts", B, 1, D, K, 0, int(bf16), 0) * B * D
         ws = torch.empty(n, dtype=torch.float32, device=dev) if n else None      # the call's own, as in _decoder_dense_fwd
         self.launches += 1                              # (two kernels in this call)
-        self._call("clt_decoder_layer_fwd", x, x.stride(0), w_op if dec.crosslayer else w_op[layer], dec.b.data[layer],
+        self._call("clt_decoder_layer_fwd", x, x.stride(0), w_op if dec.crosslayer else w_op[at], dec.b.data[at],
                    feat, recon, ws, n, B, K, D, int(bf16), self.status, s)
         return recon.view(*lead, D)
 

@@ -22,13 +22,14 @@ class _Calls:
     """In the place of the library: records what would be launched."""
 
     def __init__(self):
-        self.names = []
+        self.names, self.args = [], []
 
     def check_device(self):
         pass
 
     def call(self, name, *args):
         self.names.append(name)
+        self.args.append(args)
 
     def query(self, name, *args):
         return 0
@@ -42,8 +43,8 @@ def calls(monkeypatch):
     return rec
 
 
-def _module(kind, dev):
-    spec = synthetic.WorkloadSpec("order", 3, 64, 128, 40, kind, True, False, rank_u=8, n_outlier=1, k=4, k_aux=0)
+def _module(kind, dev, cross=True):
+    spec = synthetic.WorkloadSpec("order", 3, 64, 128, 40, kind, cross, False, rank_u=8, n_outlier=1, k=4, k_aux=0)
     batch, w, la = spec_inputs(spec)
     mod = build_module(spec, w, dev, last_active=la)
     batch = batch.to(dev)
@@ -92,6 +93,21 @@ def test_replaced_decoder_blocks_are_not_answered_with_the_old_ones(kind, replac
             dec.W_1 = torch.nn.Parameter(dec.W_1.detach() + 1)
         with pytest.raises(CltError, match="decoder block"):
             mod(acts)
+
+
+@pytest.mark.parametrize("precision", ["bf16", "fp32"])
+@pytest.mark.parametrize("tokens", [5, 200])
+@pytest.mark.parametrize("layer", [-1, 3, 7])
+def test_layers_that_do_not_exist_reach_the_library_as_null(layer, tokens, precision, calls):
+    """(which it refuses) whatever form of the call the size takes."""
+    mod, _ = _module("relu", "cpu", cross=False)
+    mod.precision = precision
+    rand = lambda n: torch.randn(tokens, n).as_subclass(_OnDevice)
+    for part, x, name in ((mod.model.encoder, rand(64), "encoder"), (mod.model.decoder, rand(128), "decoder")):
+        del calls.names[:], calls.args[:]
+        part(x, layer=layer)
+        i, = [i for i, n in enumerate(calls.names) if name in n]
+        assert any(isinstance(a, torch.Tensor) and a.dim() > 2 and a.data_ptr() == 0 for a in calls.args[i])
 
 
 @pytest.mark.parametrize("how", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))], ids=["deepcopy", "pickle"])
