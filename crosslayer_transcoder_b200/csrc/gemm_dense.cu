@@ -67,10 +67,8 @@ bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F >
 // Output tiles run `slots` at a time (one to an SM in bf16, two in fp32), so a fair share of the work is
 // total * tiles / slots k-blocks, and the launch lasts as long as its longest chain.  Parts come into question when
 // that chain is over 3/2 of the share: at 1.37 (12 layers x 9 tiles on 148 SMs, 384 blocks each) whole chains took 170
-// us and parts 200 us.  In fp32, parts of half a share keep the last wave short; in bf16 the number of parts is fitted to
-// whole rounds of the chip (12th call of a 12-layer crosslayer decoder, 257 tokens, 9 tiles: 33 parts of half a share were
-// 297 blocks on 148 SMs, a third round for one; 16 parts are one round).  Below 8 blocks a part's output costs
-// more than its products.  Then both forms are estimated (us):
+// us and parts 200 us.  Parts of half a share keep the last wave short; below 8 blocks a part's output costs more than its
+// products.  Then both forms are estimated (us):
 //   * a bf16 block takes its CTA 0.39 (staging its operands from L2), whatever the tile is filled with;
 //   * fp32: 2.2 in a 128 x 128 tile, two to an SM, 0.62 of the SM's time in a 64 x 64 tile but 0.9 of its own; small
 //     tiles are what whole chains get when the large ones are fewer than the SMs, and what parts often do not get;
@@ -84,7 +82,10 @@ bool dims_ok(int B, int L, int D, int F) { return B > 0 && L > 0 && D > 0 && F >
 //
 // Parts are also the more exact form, since accumulators take fewer terms.  Relative error against float64 over 24
 // sizes of these ranges, whole -> parts: 1.3e-4 -> 2.6e-6 (bf16, 120000 features), 8.3e-6 -> 2.7e-7 (10000), 5 to 80
-// times less in bf16 and 2 to 6 times less in fp32, nowhere more.
+// times less in bf16 and 2 to 6 times less in fp32, nowhere more.  In bf16 the error goes with a part's length (the
+// tensor-core accumulator truncates), and half a share is the longest that is taken: 257 tokens, 120000 features, 768 wide,
+// 33 parts of 58 blocks 2.9e-6 and 76 us; 16 of 119, which fill one round of the chip, would be 68 us and 6.6e-6; 49 of 39,
+// which fill three, 80 us and 1.8e-6.
 int plan_parts(GemmGeom& g, bool bf16, int sms) {
   const auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const int kb = bf16 ? tc::kBK : kSimtBK, kb_per_seg = (int)up(g.Kseg, kb);
@@ -96,29 +97,10 @@ int plan_parts(GemmGeom& g, bool bf16, int sms) {
     longest = n > longest ? n : longest;
   }
   if (longest < 32 || longest * slots * 2 <= total * tiles * 3) return 0;
-  const auto count = [&](long long part) {
-    g.kb_per_part = (int)part;
-    long long n = 0;
-    for (int z = 0; z < g.nz; ++z) n += part_count(g, z, kb_per_seg);
-    return n;
-  };
-  long long part = up(total * tiles, 2 * slots), parts;
-  if (bf16) {
-    // the shortest parts that fill 1 .. 4 rounds of the chip without beginning another; the cheapest of them
-    double best = 0;
-    long long best_part = 0;
-    for (int rounds = 1; rounds <= 4; ++rounds) {
-      long long p = up(total * tiles, rounds * slots);
-      if (p < 8) p = 8;
-      for (int i = 0; i < 64 && count(p) * tiles > rounds * slots; ++i) p += 1 + p / 64;
-      const double cost = 0.39 * p * up(count(p) * tiles, slots) + 8.0 * count(p) * g.M * g.N / 5e6;
-      if (best_part == 0 || cost < best) best = cost, best_part = p;
-    }
-    part = best_part;
-  } else if (part < 8) {
-    part = 8;
-  }
-  parts = count(part);
+  const long long half = up(total * tiles, 2 * slots), part = half < 8 ? 8 : half;
+  g.kb_per_part = (int)part;
+  long long parts = 0;
+  for (int z = 0; z < g.nz; ++z) parts += part_count(g, z, kb_per_seg);
   double whole, split;
   if (bf16) {
     whole = 0.39 * longest;
