@@ -105,13 +105,14 @@ struct Raw8 {
   }
 };
 
-// The streaming kernels over the batch (input preparation, loss forward and backward) share one shape: a thread owns 8
-// consecutive (l, d) columns, whose statistics stay in registers, and walks batch rows, kStripRows of them in flight; a
-// CTA of (32, 8) covers 256 columns and a strip of rows.  Every access is 16 bytes a lane.  They are bound by HBM; a warp
-// per (token, layer) row that fetched the statistics again for each (input preparation, loss forward), or 4 columns a
-// thread, one row at a time and 2-byte stores (loss backward) took longer
-// (fp16 batch, bf16 gradients): 4000 x 12 x 768 preparation 51 -> 39 us (5.7 TB/s), forward 55 -> 52, backward 78 -> 62;
-// 8192 x 4 x 2048 78 -> 64, 86 -> 85, 137 -> 102; 136 x 3 x 64 backward 21 -> 8.
+// Input preparation and loss backward share one shape: a thread owns 8 consecutive (l, d) columns, whose statistics stay in
+// registers, and walks batch rows, kStripRows of them in flight; a CTA of (32, 8) covers 256 columns and a strip of rows.
+// Every access is 16 bytes a lane.  A warp per (token, layer) row that fetched the statistics again for each (preparation),
+// or 4 columns a thread, one row at a time and 2-byte stores (loss backward) took longer (fp16 batch, bf16 results, inputs
+// not in L2): 4000 x 12 x 768 preparation, 147 MB, 51 -> 39 us, backward, 295 MB, 78 -> 62 (0.58 and 0.73 of the copy rate);
+// 8192 x 4 x 2048 78 -> 64, 137 -> 102; 136 x 3 x 64 backward 21 -> 8.  The loss forward, which only reads, stays with
+// columns dealt out one after another: strips took 52 us where it takes 55 (4000 x 12 x 768) but 48 against 43 with the
+// inputs in L2, twice its time at widths of 64 (65536 rows: 8 -> 19 us) and at D = 100, where columns cross a layer.
 constexpr int kStripRows = 4;
 struct Strip {
   int c, l, d, b0, b1;  // this thread's first column, its layer and place in it; this thread's first and the CTA's last row
@@ -270,62 +271,54 @@ __global__ void loss_fwd_kernel(const float* __restrict__ recon, const float* __
   }
 }
 
-// same sums (needs D % 8 == 0)
-template <class TIn, bool kAux>
-__global__ void __launch_bounds__(256)
-loss_fwd_vec_kernel(const float* __restrict__ recon, const float* __restrict__ aux, const TIn* __restrict__ batch,
-                    const float* __restrict__ mu, const float* __restrict__ sd, float* __restrict__ acc, int B, int L,
-                    int D, int rows_per_cta) {
-  const Strip t(B, D, rows_per_cta);
-  const int LD = L * D;
-  constexpr int R = kAux ? 2 : kStripRows;
+// same sums, 8 consecutive (l, d) columns per thread (needs L*D % 8 == 0)
+template <class TIn>
+__global__ void loss_fwd_vec_kernel(const float* __restrict__ recon, const float* __restrict__ aux,
+                                    const TIn* __restrict__ batch, const float* __restrict__ mu,
+                                    const float* __restrict__ sd, float* __restrict__ acc, int B, int L, int D) {
+  const long long LD = (long long)L * D;
+  const long long total = (long long)B * LD / 8;
   float s0 = 0.f, s1 = 0.f;
-  if (t.c < LD) {
-    float m[8], sv[8];
-    load8<float>(mu + t.c, m);
-    load8<float>(sd + t.c, sv);
-    const TIn* yp = batch + LD + t.c;
-    for (int b = t.b0; b < t.b1; b += 8 * R) {
-      RawIn<TIn> raw[R];
-      RawIn<float> rec[R], ax[kAux ? R : 1];
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long e = i * 8;
+    const long long c = e % LD, b = e / LD;
+    float y[8], m[8], sdv[8], r[8];
+    load8<TIn>(batch + (b * 2 + 1) * LD + c, y);
+    load8<float>(mu + c, m);
+    load8<float>(sd + c, sdv);
+    load8<float>(recon + e, r);
+    float diff[8];
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-        if (b + 8 * i < t.b1) {
-          const long long o = (long long)(b + 8 * i) * LD;
-          raw[i].load(yp + 2 * o);
-          rec[i].load(recon + o + t.c);
-          if constexpr (kAux) ax[i].load(aux + o + t.c);
-        }
+    for (int q = 0; q < 8; ++q) {
+      diff[q] = r[q] - (y[q] - m[q]) / sdv[q];
+      s0 = fmaf(diff[q], diff[q], s0);
+    }
+    if (aux != nullptr) {
+      float a[8];
+      load8<float>(aux + e, a);
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-        if (b + 8 * i < t.b1) {
-          float y[8], r[8], a[8];
-          raw[i].get(y);
-          rec[i].get(r);
-          if constexpr (kAux) ax[i].get(a);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const float diff = r[q] - (y[q] - m[q]) / sv[q];
-            s0 = fmaf(diff, diff, s0);
-            if constexpr (kAux) {
-              const float ad = a[q] + diff, sq = ad * ad;
-              s1 += (sq == sq) ? sq : 0.f;
-            }
-          }
-        }
+      for (int q = 0; q < 8; ++q) {
+        const float ad = a[q] + diff[q];
+        const float sq = ad * ad;
+        s1 += (sq == sq) ? sq : 0.f;
+      }
     }
   }
   s0 = warp_sum(s0);
   s1 = warp_sum(s1);
-  __shared__ float sh[2][8];
-  if (threadIdx.x == 0) sh[0][threadIdx.y] = s0, sh[1][threadIdx.y] = s1;
+  __shared__ float sh[2][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) sh[0][w] = s0, sh[1][w] = s1;
   __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    s0 = s1 = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) s0 += sh[0][w], s1 += sh[1][w];
-    atomicAdd(acc + 0, s0);
-    if (kAux) atomicAdd(acc + 1, s1);
+  if (w == 0) {
+    const int nw = blockDim.x >> 5;
+    s0 = warp_sum(lane < nw ? sh[0][lane] : 0.f);
+    s1 = warp_sum(lane < nw ? sh[1][lane] : 0.f);
+    if (lane == 0) {
+      atomicAdd(acc + 0, s0);
+      if (aux != nullptr) atomicAdd(acc + 1, s1);
+    }
   }
 }
 
@@ -334,17 +327,14 @@ int loss_fwd(const float* recon, const float* aux, const void* batch, int in_dty
   if (B <= 0) return 0;
   const long long total = (long long)B * L * D;
   const int threads = 256;
-  const bool vec = strip_ok(B, L, D) &&
+  const bool vec = ((long long)L * D) % 8 == 0 &&
                    ((uintptr_t)recon | (uintptr_t)aux | (uintptr_t)batch | (uintptr_t)mu | (uintptr_t)sd) % 16 == 0;
-  const int blocks = (int)min((total + threads - 1) / threads, (long long)148 * 8);
-  const int rows = vec ? strip_rows(B, L * D) : 0;
-  const dim3 grid = vec ? strip_grid(B, L * D, rows) : dim3(blocks), strip(32, 8);
-#define CLT_LF(TI)                                                                                                   \
-  if (vec && aux != nullptr)                                                                                         \
-    loss_fwd_vec_kernel<TI, true><<<grid, strip, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D, rows);  \
-  else if (vec)                                                                                                      \
-    loss_fwd_vec_kernel<TI, false><<<grid, strip, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D, rows); \
-  else                                                                                                               \
+  const long long work = vec ? total / 8 : total;
+  const int blocks = (int)min((work + threads - 1) / threads, (long long)148 * 8);
+#define CLT_LF(TI)                                                                                               \
+  if (vec)                                                                                                       \
+    loss_fwd_vec_kernel<TI><<<blocks, threads, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D);      \
+  else                                                                                                           \
     loss_fwd_kernel<TI><<<blocks, threads, 0, s>>>(recon, aux, (const TI*)batch, mu, sd, acc, B, L, D)
   if (in_dtype == 0) {
     CLT_LF(float);

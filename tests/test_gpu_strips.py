@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,L,D", [(1, 1, 8), (9, 3, 88), (31, 2, 128), (65, 5, 72), (300, 2, 264), (2049, 1, 16),
-                                   (33, 3, 20)])
+                                   (33, 3, 20), (31, 2, 20), (9, 12, 100)])
 def test_against_float64(B, L, D, dtype, out):
     g = torch.Generator(device="cuda:0").manual_seed(B + D)
     r = lambda *s: torch.randn(*s, generator=g, device="cuda:0")
@@ -45,3 +45,23 @@ def test_against_float64(B, L, D, dtype, out):
         if a is not None:
             assert bool(((da.transpose(0, 1).double() - ga).abs() <= tol * mag).all())
         assert bool(((db.double() - (gr + ga).sum(0)).abs() <= 2.0 ** -20 * 2 * mag.sum(0)).all())
+
+
+def test_more_rows_than_a_grid_of_short_strips():
+    """600000 rows: strips of 8 would be more than a grid has in y.  Rows of one constant, so that the sums are known."""
+    B, L, D, s = 600000, 1, 8, stream_ptr()
+    batch, mu, sd = torch.full((B, 2, L, D), 3.0, device="cuda:0"), torch.ones(L, D, device="cuda:0"), \
+        torch.full((L, D), 2.0, device="cuda:0")
+    recon, aux = torch.full((B, L, D), 1.5, device="cuda:0"), torch.full((B, L, D), -1.0, device="cuda:0")
+    xn, acc = torch.empty(L, B, D, device="cuda:0"), torch.zeros(2, device="cuda:0")
+    lib().call("clt_prep_input", batch, 0, mu, sd, xn, 0, B, L, D, s)
+    assert bool((xn == 1.0).all())
+    lib().call("clt_loss_fwd", recon, aux, batch, 0, mu, sd, acc, B, L, D, s)
+    # diff = 0.5, aux + diff = -0.5; fp32 sums of 4.8 million equal terms over 148 x 8 x 256 threads
+    assert torch.allclose(acc, torch.full_like(acc, 0.25 * B * L * D), rtol=1e-5)
+    dr, da, db = torch.empty_like(xn), torch.empty_like(xn), torch.zeros(L, D, device="cuda:0")
+    lib().call("clt_loss_bwd", recon, aux, batch, 0, mu, sd, None, 0.25, dr, da, 0, db, B, L, D, s)
+    n = B * L * D
+    assert torch.allclose(da, torch.full_like(da, -0.25 / n), rtol=1e-6)
+    assert torch.allclose(dr, torch.full_like(dr, 0.75 / n), rtol=1e-6)
+    assert torch.allclose(db, torch.full_like(db, 0.5 / D), rtol=1e-4)
