@@ -705,9 +705,17 @@ int loss_bwd(const float* recon, const float* aux, const void* batch, int in_dty
   const int rows_per_cta = 256;
   const bool vec = D % 4 == 0 && ((uintptr_t)recon | (uintptr_t)aux | (uintptr_t)mu | (uintptr_t)sd) % 16 == 0;
   dim3 grid(vec ? (LD / 4 + 31) / 32 : (LD + 31) / 32, (B + rows_per_cta - 1) / rows_per_cta), block(32, 8);
-  const bool strips = vec && strip_ok(B, L, D) && ((uintptr_t)batch | (uintptr_t)drecon | (uintptr_t)daux) % 16 == 0;
-  // fp32 steps add the bias gradient up in the order in which the kernels below do (256 rows to a CTA): what follows
-  // from its last bits reaches thresholds
+  // Strips read and write 16 bytes a lane with more rows in flight, but
+  //   * a CTA covers 256 columns: narrower rows leave its lanes idle, which short batches hide (3 x 64: 21 -> 8 us) and long
+  //     ones do not (65536 x 64: 21 -> 25 us, with aux 23 -> 34);
+  //   * fp32 steps keep strips of 256 rows, the kernels' below, so that as long as two strips hold the batch the bias
+  //     gradient has the same bits (what follows from them reaches thresholds; more strips add up in any order, here as
+  //     there).  With 8 columns a thread that is half the CTAs: 512 x 12 x 768 17 -> 19 us, with aux 25 -> 29, from L2; where
+  //     there is one for nearly every SM, or two with aux, strips are faster (4000 x 2304 29 -> 21, 2047 x 12 x 768 42 -> 33;
+  //     with aux 8192 x 4 x 2048 219 -> 199, but 2047 x 12 x 768 64 -> 70).
+  const bool fill = (long long)((LD / 8 + 31) / 32) * ((B + 255) / 256) >= (aux != nullptr ? 2 * 148 : 128);
+  const bool strips = vec && strip_ok(B, L, D) && ((uintptr_t)batch | (uintptr_t)drecon | (uintptr_t)daux) % 16 == 0 &&
+                      (out_bf16 ? LD >= 256 || B <= 32768 : LD >= 256 && fill);
   const int rows = !strips ? 0 : out_bf16 ? strip_rows(B, LD) : 256;
   const dim3 sgrid = strips ? strip_grid(B, LD, rows) : dim3(1);
 #define CLT_LB(TI, TO)                                                                                            \

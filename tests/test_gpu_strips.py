@@ -8,11 +8,13 @@ from crosslayer_transcoder_b200._lib import DTYPE_CODE, lib, stream_ptr
 pytestmark = pytest.mark.gpu
 
 
-# 256 columns to a CTA, strips of 8 to 64 rows (256 in fp32), 2 or 4 rows in flight per thread
+# 256 columns to a CTA, strips of 8 to 64 rows (256 in fp32, where that gives two CTAs to an SM), 2 or 4 rows in flight per
+# thread; long batches of narrow rows
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,L,D", [(1, 1, 8), (9, 3, 88), (31, 2, 128), (65, 5, 72), (300, 2, 264), (2049, 1, 16),
-                                   (33, 3, 20), (31, 2, 20), (9, 12, 100)])
+                                   (33, 3, 20), (31, 2, 20), (9, 12, 100), (2305, 12, 768),
+                                   (32769, 1, 248), (32768, 1, 248)])
 def test_against_float64(B, L, D, dtype, out):
     g = torch.Generator(device="cuda:0").manual_seed(B + D)
     r = lambda *s: torch.randn(*s, generator=g, device="cuda:0")
@@ -65,3 +67,24 @@ def test_more_rows_than_a_grid_of_short_strips():
     assert torch.allclose(da, torch.full_like(da, -0.25 / n), rtol=1e-6)
     assert torch.allclose(dr, torch.full_like(dr, 0.75 / n), rtol=1e-6)
     assert torch.allclose(db, torch.full_like(db, 0.5 / D), rtol=1e-4)
+
+
+@pytest.mark.parametrize("B", [256, 300, 512])
+def test_fp32_bias_gradient_has_one_order_up_to_two_strips(B):
+    """A batch that does not start on 16 bytes goes to the kernel with 4 columns a thread: the same bits."""
+    L, D, s = 16, 2368 * (2 if B == 256 else 1), stream_ptr()
+    assert -(-L * D // 256) * -(-B // 256) >= 2 * 148
+    g = torch.Generator(device="cuda:0").manual_seed(B)
+    r = lambda *n: torch.randn(*n, generator=g, device="cuda:0")
+    mu, sd, recon, aux = 0.3 * r(L, D), 0.5 + r(L, D).abs(), r(B, L, D), r(B, L, D)
+    store = r(B * 2 * L * D + 1).half()
+    for a in (None, aux):
+        got = []
+        for off in (0, 1):
+            batch = store[off:off + B * 2 * L * D] if off else store[1:].clone()
+            assert (batch.data_ptr() % 16 != 0) == bool(off)
+            dr, da, db = torch.empty(L, B, D, device="cuda:0"), torch.empty(L, B, D, device="cuda:0"), torch.zeros(L, D, device="cuda:0")
+            lib().call("clt_loss_bwd", recon, a, batch, 1, mu, sd, None, 0.03 if a is not None else 0.0, dr,
+                       da if a is not None else None, 0, db, B, L, D, s)
+            got.append((dr, db, da if a is not None else dr))
+        assert all(torch.equal(x, y) for x, y in zip(*got))
