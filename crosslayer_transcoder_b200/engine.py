@@ -707,8 +707,11 @@ class StepEngine:
         s = stream_ptr()
         at = slice(layer, layer + 1)        # empty, which the library refuses, where there is no such layer
         xn = torch.empty(1, B, D, dtype=T, device=dev)
-        if bf16 and B * F >= 16384:
-            # the contraction's epilogue writes the result; fewer values than a tile's are launch latency either way
+        if bf16 and F >= 256:
+            # The contraction's epilogue writes the result: two launches and one entry into the library instead of three of
+            # each, from one token on (768 x 10000: 1 token 24.6 -> 22.5 us alone, 16.5 -> 14.4 among others; 32 tokens 18.5
+            # -> 16.4; 2 x 2304 x 16384 25.8 -> 23.1).  Layers narrower than a tile would gain as well (15 -> 10); nothing
+            # but the tests, which count the launches, has them.
             out = torch.empty(B, F, dtype=torch.float32, device=dev)
             self.launches += 1                          # (two kernels in this call)
             self._call("clt_encoder_layer_fwd", x, DTYPE_CODE[x.dtype], self._operand(enc.W, bf16)[at],
@@ -756,7 +759,7 @@ class StepEngine:
         recon = torch.empty(B, D, dtype=torch.float32, device=dev)
         n = lib().query("clt_decoder_dense_parts", B, 1, D, K, 0, int(bf16), 0) * B * D
         ws = torch.empty(n, dtype=torch.float32, device=dev) if n else None      # the call's own, as in _decoder_dense_fwd
-        self.launches += 1                              # (two kernels in this call)
+        self.launches += 2 if n else 1                  # (two kernels in this call, three where parts are summed)
         self._call("clt_decoder_layer_fwd", x, x.stride(0), w_op if dec.crosslayer else w_op[at], dec.b.data[at],
                    feat, recon, ws, n, B, K, D, int(bf16), self.status, s)
         return recon.view(*lead, D)
