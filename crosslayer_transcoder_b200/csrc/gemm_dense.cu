@@ -190,6 +190,7 @@ int clt_encoder_layer_fwd(const void* x, int in_dtype, const void* W_enc, const 
                           int D, int F, int* status, clt_stream_t stream) {
   CLT_CHECK_ARG(dims_ok(B, 1, D, F), "encoder_layer_fwd: bad dims B=%d D=%d F=%d", B, D, F);
   CLT_CHECK_ARG(x && W_enc && xn && out && status, "encoder_layer_fwd: null pointer");
+  CLT_CHECK_ARG((uintptr_t)out % 16 == 0, "encoder_layer_fwd: out must be 16-byte aligned");
   if (int rc = prep_input(x, in_dtype, nullptr, nullptr, xn, 1, B, 1, D, 1, (cudaStream_t)stream)) return rc;
   GemmGeom g{kBatched, B, F, D, 1, 1};
   Operand a{xn, 1, B, D, 1}, b{W_enc, 0, F, D, 1};

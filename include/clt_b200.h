@@ -61,8 +61,8 @@ int clt_encoder_fwd_act(const void* xn, const void* W_enc, const float* b_enc, c
 int clt_encoder_fwd_store(const void* xn, const void* W_enc, void* z_out, int B, int L, int D, int F, int bf16,
                           int* status, clt_stream_t stream);
 
-/* Encoder.forward_layer (clt.py:134-145) on bf16 operands: out [B,F] fp32 = round_T(T(x) W_enc) + b_enc (NULL: none) for
- * x [B,D] of type in_dtype and one layer's W_enc [D,F]; xn [B,D] in T is scratch. */
+/* Encoder.forward_layer (clt.py:134-145) on bf16 operands: out [B,F] fp32 (16-byte aligned) = round_T(T(x) W_enc) + b_enc
+ * (NULL: none) for x [B,D] of type in_dtype and one layer's W_enc [D,F]; xn [B,D] in T is scratch. */
 int clt_encoder_layer_fwd(const void* x, int in_dtype, const void* W_enc, const float* b_enc, void* xn, float* out, int B,
                           int D, int F, int* status, clt_stream_t stream);
 /* Decoder.forward_layer, CrosslayerDecoder.forward_layer (clt.py:216-231, 304-317): clt_import_rows, then

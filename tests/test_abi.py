@@ -26,6 +26,15 @@ def test_argument_errors_do_not_launch():
     assert rc != 0 and "bad dims" in L.last_error()
 
 
+def test_fused_outputs_that_are_not_aligned_are_refused():
+    """Epilogues store whole vectors of a row: an output that does not start on one is an argument error, not an access."""
+    L, one = _lib.lib(), 1 << 20        # (addresses that nothing looks at)
+    rc = L.cdll.clt_encoder_layer_fwd(one, 0, one, one, one, one + 4, 8, 64, 256, one, None)
+    assert rc != 0 and "aligned" in L.last_error()
+    rc = L.cdll.clt_select_topk_export(one, one, one, one, one, one + 16, 8, 2, 256, 4, 1, None)
+    assert rc != 0 and "aligned" in L.last_error()
+
+
 def _calls_in(path):
     """(entry point, number of arguments, line) of every ``_call("clt_...", ...)`` / ``lib().call("clt_...", ...)``
     in a Python source file, with the arguments counted at nesting depth 0."""
