@@ -602,7 +602,9 @@ class StepEngine:
         tensors of the return value are written by ``clt_act_export`` or ``clt_select_topk_export``, else by
         ``clt_export_blf`` and ``clt_scatter_features``.  The sparse decoder takes the CTA form of the gather at every size
         (``module.decoder_gather_warp`` is a switch of the training step): the warp form took 358 us where it
-        takes 245 (1000 tokens, 12 layers, 16 entries of 768 columns).  No
+        takes 245 (1000 tokens, 12 layers, 16 entries of 768 columns).  Where several pre-activations equal the k-th largest
+        (biases all alike, as at initialisation, in bf16) a TopK of up to 8192 features may keep other ones of them than the
+        training step.  No
         autograd graph is built.  On feature shards the partial reconstructions are summed over the ranks;
         the returned features are the rank's slice, and nonlinearities that rank across the whole feature
         axis (TopK, BatchTopK) are refused there."""

@@ -197,7 +197,8 @@ int clt_select_topk(const void* z, const float* b_enc, int* idx_out, float* val_
 
 /* clt_select_topk, clt_export_blf and clt_scatter_features of the inference forward in one sweep of z: pre_out [B,L,F] =
  * z + b_enc, features_out [B,L,F] = the selected values, 0 elsewhere (both fp32, 32-byte aligned).  F a multiple of 8,
- * 1 <= k <= 256; the entries of a row come largest value first. */
+ * 1 <= k <= 256; the entries of a row come largest value first.  Of values equal to the k-th, which ones are taken is left
+ * open here as in clt_select_topk, and for rows of up to 8192 features need not be the ones that it takes. */
 int clt_select_topk_export(const void* z, const float* b_enc, int* idx_out, float* val_out, float* pre_out,
                            float* features_out, int B, int L, int F, int k, int bf16, clt_stream_t stream);
 
