@@ -130,9 +130,9 @@ import_rows_kernel(const float* __restrict__ src, long long ld, T* __restrict__ 
   }
 }
 
-// grid of the kernels above: about 16 CTAs per SM, fewer rows per CTA rather than fewer CTAs
-inline dim3 row_grid(int B, int L, long long F, int V) {
-  const long long gx = (F + 256ll * V - 1) / (256ll * V);
+// grid of these kernels for CTAs `wide` columns wide: about 16 CTAs per SM, fewer rows per CTA rather than fewer CTAs
+inline dim3 row_grid(int B, int L, long long F, long long wide) {
+  const long long gx = (F + wide - 1) / wide;
   long long gy = (148ll * 16 + gx * L - 1) / (gx * L);
   if (gy > B) gy = B;
   return dim3((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535), (unsigned)L);
@@ -140,18 +140,18 @@ inline dim3 row_grid(int B, int L, long long F, int V) {
 template <class T>
 int launch_import(const float* src, long long ld, void* dst, int B, int L, long long F, cudaStream_t s) {
   if (F % 8 == 0 && ld % 8 == 0 && aligned32(src) && aligned32(dst))
-    import_rows_kernel<T, 8><<<row_grid(B, L, F, 8), 256, 0, s>>>(src, ld, (T*)dst, B, F);
+    import_rows_kernel<T, 8><<<row_grid(B, L, F, 256 * 8), 256, 0, s>>>(src, ld, (T*)dst, B, F);
   else
-    import_rows_kernel<T, 1><<<row_grid(B, L, F, 1), 256, 0, s>>>(src, ld, (T*)dst, B, F);
+    import_rows_kernel<T, 1><<<row_grid(B, L, F, 256), 256, 0, s>>>(src, ld, (T*)dst, B, F);
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 template <class T>
 int launch_export(const void* src, const float* bias, float* out, int B, int L, long long F, cudaStream_t s) {
   if (F % 8 == 0 && aligned32(src) && aligned32(out))
-    export_blf_kernel<T, 8><<<row_grid(B, L, F, 8), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
+    export_blf_kernel<T, 8><<<row_grid(B, L, F, 256 * 8), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
   else
-    export_blf_kernel<T, 1><<<row_grid(B, L, F, 1), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
+    export_blf_kernel<T, 1><<<row_grid(B, L, F, 256), 256, 0, s>>>((const T*)src, bias, out, B, L, F);
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
@@ -160,28 +160,29 @@ int launch_act_export(const void* z, const float* bias, const float* theta, floa
                       int B, int L, long long F, cudaStream_t s) {
   if (F % 8 == 0 && aligned32(z) && aligned32(pre) && aligned32(feat) && aligned32(features))
     act_export_kernel<T, 8>
-        <<<row_grid(B, L, F, 8), 256, 0, s>>>((const T*)z, bias, theta, pre, (T*)feat, features, B, L, F);
+        <<<row_grid(B, L, F, 256 * 8), 256, 0, s>>>((const T*)z, bias, theta, pre, (T*)feat, features, B, L, F);
   else
     act_export_kernel<T, 1>
-        <<<row_grid(B, L, F, 1), 256, 0, s>>>((const T*)z, bias, theta, pre, (T*)feat, features, B, L, F);
+        <<<row_grid(B, L, F, 256), 256, 0, s>>>((const T*)z, bias, theta, pre, (T*)feat, features, B, L, F);
   CLT_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
 
-// out[b, l, d] = recon[b, l, d] * sd[l, d] + mu[l, d].  HBM-bound: blockIdx.x covers 256 V columns of the L D of a row,
-// blockIdx.y walks rows, so the statistics stay in registers and an element costs no 64-bit division (1000 x 12 x 768:
-// 33 -> 18 us, 4.1 TB/s; 1500 x 12 x 2304: 112 -> 64 us, 5.2 TB/s).  V = 4: 16-byte accesses.
+// out[b, l, d] = recon[b, l, d] * sd[l, d] + mu[l, d].  A CTA's x covers V columns a thread of the L D of a row, its y (where
+// rows are narrower than 256 threads) and blockIdx.y walk rows, so that the statistics stay in registers and an element
+// costs no 64-bit division (inputs not in L2: 1000 x 12 x 768 33 -> 18 us, 4.1 TB/s; 1500 x 12 x 2304 112 -> 64 us, 5.2
+// TB/s).  V = 4: 16-byte accesses.
 template <int V>
 __global__ void __launch_bounds__(256)
 destandardize_kernel(const float* __restrict__ recon, const float* __restrict__ mu, const float* __restrict__ sd,
                      float* __restrict__ out, int B, long long LD) {
-  const long long c = (blockIdx.x * 256ll + threadIdx.x) * V;
+  const long long c = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * V;
   if (c >= LD) return;
   float m[V], d[V];
 #pragma unroll
   for (int q = 0; q < V; ++q) m[q] = __ldg(mu + c + q), d[q] = __ldg(sd + c + q);
 #pragma unroll 4
-  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+  for (long long b = blockIdx.y * blockDim.y + threadIdx.y; b < B; b += gridDim.y * blockDim.y) {
     const long long i = b * LD + c;
     if constexpr (V == 4) {
       const float4 r = *reinterpret_cast<const float4*>(recon + i);
@@ -191,6 +192,18 @@ destandardize_kernel(const float* __restrict__ recon, const float* __restrict__ 
       out[i] = fmaf(recon[i], d[0], m[0]);
     }
   }
+}
+template <int V>
+int launch_destandardize(const float* recon, const float* mu, const float* sd, float* out, int B, long long LD,
+                         cudaStream_t s) {
+  const long long cols = (LD + V - 1) / V;
+  int x = 256;
+  while (x > 1 && x / 2 >= cols) x /= 2;
+  const dim3 block(x, 256 / x);
+  const dim3 grid = row_grid((B + (int)block.y - 1) / (int)block.y, 1, LD, x * V);
+  destandardize_kernel<V><<<grid, block, 0, s>>>(recon, mu, sd, out, B, LD);
+  CLT_CHECK_CUDA(cudaGetLastError());
+  return 0;
 }
 
 // dense[token, l, idx] = val for every valid entry of the per-layer lists idx / val [L, npl]; the token of
@@ -266,13 +279,8 @@ int clt_destandardize(const float* recon, const float* mu, const float* sd, floa
   CLT_CHECK_ARG(recon && mu && sd && out && B > 0 && L > 0 && D > 0, "destandardize: bad arguments");
   const long long LD = (long long)L * D;
   const int V = LD % 4 == 0 && ((uintptr_t)recon | (uintptr_t)out) % 16 == 0 ? 4 : 1;
-  const dim3 grid = row_grid(B, 1, LD, V);
-  if (V == 4)
-    destandardize_kernel<4><<<grid, 256, 0, (cudaStream_t)stream>>>(recon, mu, sd, out, B, LD);
-  else
-    destandardize_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(recon, mu, sd, out, B, LD);
-  CLT_CHECK_CUDA(cudaGetLastError());
-  return 0;
+  return V == 4 ? launch_destandardize<4>(recon, mu, sd, out, B, LD, (cudaStream_t)stream)
+                : launch_destandardize<1>(recon, mu, sd, out, B, LD, (cudaStream_t)stream);
 }
 
 int clt_scatter_features(const int* idx, const float* val, const int* etok, float* dense, int B, int L, int F, int k,

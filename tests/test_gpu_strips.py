@@ -88,3 +88,19 @@ def test_fp32_bias_gradient_has_one_order_up_to_two_strips(B):
                        da if a is not None else None, 0, db, B, L, D, s)
             got.append((dr, db, da if a is not None else dr))
         assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
+# one CTA's columns of a row and more, rows narrower than a CTA (powers of two and not), 16-byte rows and others
+@pytest.mark.parametrize("B,L,D", [(1, 1, 1), (5, 1, 4), (1001, 1, 7), (257, 1, 16), (3000, 1, 100), (70000, 2, 8), (33, 3, 33),
+                                   (129, 1, 1020), (7, 2, 512), (9, 1, 1028), (300, 12, 768)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_destandardize(B, L, D, offset):
+    g = torch.Generator(device="cuda:0").manual_seed(B + D)
+    flat = torch.randn(B * L * D + offset, generator=g, device="cuda:0")[offset:]       # (a base that is not on 16 bytes)
+    mu, sd = torch.randn(L, D, generator=g, device="cuda:0"), torch.rand(L, D, generator=g, device="cuda:0") + 0.1
+    out = torch.full((B * L * D + 8,), float("nan"), device="cuda:0")
+    lib().call("clt_destandardize", flat, mu, sd, out, B, L, D, stream_ptr())
+    want = flat.view(B, L, D).double() * sd.double() + mu.double()
+    # one rounding of the exact value
+    assert bool(((out[:-8].view(B, L, D).double() - want).abs() <= 2.0 ** -24 * 1.001 * want.abs() + 1e-45).all())
+    assert bool(out[-8:].isnan().all())                                                 # and nothing behind the end
