@@ -229,9 +229,10 @@ __device__ __forceinline__ void store_rows32_scalar(unsigned char* stage, float*
 }
 
 // Store a warp's sub-tile through `stage`, in 16-byte pieces when the 32 columns are all inside the matrix and rows are
-// 16-byte aligned; others lane by lane with guards.  kOdd: fp32 rows may end anywhere (feature counts do; widths hardly
-// ever, and for them the second way through `stage` cost the CUDA-core kernel 3 % in spilled registers).  `row0` is the
-// warp's first row.
+// 16-byte aligned; others lane by lane with guards.  kOdd: fp32 rows may end anywhere, as rows of features do; the epilogues
+// of pre-activations, features and their gradients have it.  Those whose rows are reconstructions or weights do not: the
+// second way through `stage` cost them 3 % on the CUDA cores, in spilled registers, whatever the row's length, and of them
+// only the encoder's weight gradient has rows of features.  `row0` is the warp's first row.
 template <class T, bool kOdd = false>
 __device__ __forceinline__ void store_tile(unsigned char* stage, T* mat, size_t ld, int row0, int row, bool row_ok,
                                            int M, int n0, int N, bool aligned, const float (&v)[32]) {

@@ -453,11 +453,12 @@ select_topk_warp_kernel(const T* __restrict__ z, const float* __restrict__ b_enc
 // kExport (inference): every pre-activation is written token-major on the way, and the token-major features, which are
 // zero but for the k selected.  Bound by the writes (4.7 to 5.8 TB/s in all) where the selection alone is bound by
 // instruction issue, so that the selection comes for free: rows of bf16 against the selection, the layout kernel, the zero
-// fill and the scatter, 12 x 1000 x 10000 (k = 16) 355 -> 256 us, 12 x 4000 x 32768 (k = 32) 3593 -> 2724 us; rows that
-// the two-sweep kernels select from (clt_select_topk) gain as well: 12 x 1000 x 4096, k = 32 169 -> 122 (k = 64 361 -> 151),
-// x 1024, k = 16 62 -> 56, x 256, k = 8 145 -> 37; x 512, k = 16 loses 5 of 45 us.  Values equal to the k-th are kept in the
-// order in which they came to the list, which is another one there: a training step and an inference call may then keep
-// different ones of such features.  With a bias of its own for every feature there are none in practice.
+// fill and the scatter, 12 x 1000 x 10000 (k = 16) 355 -> 256 us, 12 x 4000 x 32768 (k = 32) 3593 -> 2724 us.  Rows that
+// the two-sweep kernels select from (clt_select_topk) gain as well where they are long or the batch is short: 12 x 1000 x
+// 4096, k = 32 171 -> 121, x 256, k = 8 145 -> 37 us; the caller's rule and its measurements are in engine.py.  Values
+// equal to the k-th are kept in the order in which they came to the list, which is another one there: a training step and
+// an inference call may then keep different ones of such features.  With a bias of its own for every feature there are none
+// in practice.
 // ---------------------------------------------------------------------------------------
 constexpr int kStreamWarps = 8;
 constexpr int kStreamMinF = 2048;   // shorter rows keep the one-warp-per-row two-sweep kernel

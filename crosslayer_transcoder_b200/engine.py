@@ -590,6 +590,23 @@ class StepEngine:
                     l0_src=(feat, 2 if bf16 else 0, B * F))
 
     # ------------------------------------------------------------------ inference forward
+    @staticmethod
+    def _one_sweep(F: int, k: int, rows: int) -> bool:
+        """TopK inference: does the streaming selection write both token-major results on its way
+        (``clt_select_topk_export``), which saves a second sweep of z and a pass of zeros?  Where ``clt_select_topk``
+        would take the two-sweep warp kernel, that one is lighter on short rows, most of all on those that end inside
+        a step of 256 columns, unless the passes are little more than their launches.  Three passes -> one sweep, us:
+        12000 rows, k = 16: 512 45 -> 50, 768 55 -> 53, 1016 66 -> 73, 1528 79 -> 93, 2040 97 -> 99, 1024 62 -> 56,
+        3000 129 -> 101, 8192 287 -> 198; k = 48: 640 62 -> 109, 2040 112 -> 168, 2048 109 -> 100, 3000 147 -> 131;
+        1200 rows: 1016 k = 24 25 -> 23, k = 32 25 -> 26, 512 k = 48 23 -> 16."""
+        if F % 8 != 0 or not 0 < k <= 256:
+            return False
+        if not (512 <= F <= 8192 and k <= 64):                      # not the warp kernel's rows
+            return True
+        if F >= 2560:
+            return True
+        return (F >= 1024 or rows <= 4096) if F % 256 == 0 else (k <= 24 and rows <= 2048)
+
     @torch.no_grad()
     def infer(self, acts: torch.Tensor):
         """``(pre_actvs [B,L,F], features [B,L,F], recons_norm [B,L,D], recons [B,L,D])`` of
@@ -639,9 +656,7 @@ class StepEngine:
         z = torch.empty(L, B, F, dtype=T, device=dev)
         self._call("clt_encoder_fwd_store", xn, self._operand(enc.W, bf16), z, B, L, D, F, int(bf16), self.status, s)
         pre_actvs = torch.empty(B, L, F, dtype=torch.float32, device=dev)
-        # TopK: the streaming selection writes both token-major results on its way, which saves a second sweep of z and
-        # a pass of zeros, at every row length that it takes (measurements at its kernel, csrc/select.cu)
-        one_sweep = kind == "topk" and F % 8 == 0 and 0 < int(nl.k) <= min(F, 256)
+        one_sweep = kind == "topk" and int(nl.k) <= F and self._one_sweep(F, int(nl.k), L * B)
         if kind not in ("jumprelu", "relu") and not one_sweep:
             self._call("clt_export_blf", z, enc.b.data, pre_actvs, B, L, F, int(bf16), s)
         features = torch.empty(B, L, F, dtype=torch.float32, device=dev)

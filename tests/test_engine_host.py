@@ -110,6 +110,25 @@ def test_layers_that_do_not_exist_reach_the_library_as_null(layer, tokens, preci
         assert any(isinstance(a, torch.Tensor) and a.dim() > 2 and a.data_ptr() == 0 for a in calls.args[i])
 
 
+# the lines of the rule: width of a step, lengths and batches from which one sweep is the faster form
+@pytest.mark.parametrize("F,k,tokens,one", [(248, 64, 900, True), (256, 256, 5, True), (260, 8, 5, False), (512, 16, 1400, False),
+                                            (512, 16, 1300, True), (520, 16, 700, False), (520, 16, 600, True),
+                                            (520, 32, 5, False), (520, 65, 1400, True), (1024, 64, 1400, True),
+                                            (1032, 16, 1400, False), (2552, 16, 1400, False), (2560, 64, 1400, True),
+                                            (2568, 64, 1400, True), (8200, 64, 5, True), (8192, 257, 5, False)])
+def test_forms_of_the_topk_inference(F, k, tokens, one, calls):
+    L, D = 3, 64
+    spec = synthetic.WorkloadSpec("forms", L, D, F, 16, "topk", False, True, rank_u=8, n_outlier=1, k=k, k_aux=0)
+    batch, w, la = spec_inputs(spec)
+    mod = build_module(spec, w, "cpu", last_active=la)
+    mod.model.initialize_standardizers(batch)
+    with torch.no_grad():
+        mod(torch.zeros(tokens, L, D).as_subclass(_OnDevice))
+    three = ["clt_export_blf", "clt_select_topk", "clt_scatter_features"]
+    got = [n for n in calls.names if n in three or n == "clt_select_topk_export"]
+    assert got == (["clt_select_topk_export"] if one else three)
+
+
 @pytest.mark.parametrize("how", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))], ids=["deepcopy", "pickle"])
 def test_module_that_has_run_can_be_copied(how, monkeypatch):
     """Weight averaging copies a module, spawned workers pickle it: the engine holds nothing of the loaded library."""
